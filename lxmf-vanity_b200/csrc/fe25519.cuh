@@ -5,8 +5,8 @@
 // (8 little-endian 32-bit words) standing for x mod p.  2^256 = 38 (mod p),
 // so sums and products fold their overflow back with a multiply by 38; only
 // fe_canon maps to the canonical [0, p) encoding (the reference's
-// fe_to_words, common.h:145-174).  Multiplies are 32x32->64 IMAD chains with
-// explicit carries (fe25519_ptx.cuh, generated by gen_fe_ptx.py).
+// fe_to_words, common.h:145-174).  Multiplies are chains of 32 x 32 + 64 multiply-adds
+// with carry (fe25519_ptx.cuh, generated by gen_fe_ptx.py).
 #pragma once
 #include <cstdint>
 
@@ -16,18 +16,22 @@ struct __align__(16) fe {
 
 #include "fe25519_ptx.cuh"
 
-// The multiply and the square are out of line: one body each in the binary,
-// reached by a call.  Measured on B200 against the bodies inlined at every
-// call site: the grouped walk +1.5% and the pool kernel +2% (smaller loops for
-// the instruction caches), the x-only walk -2.3% (four times the multiplies
-// per key, so the calls cost more than the code size saves).
-static __device__ __noinline__ fe fe_mul(const fe& a, const fe& b) {
+// Both are bound by the multiply-add pipe: a multiply is 72 aligned
+// 32 x 32 + 64 multiply-adds (half rate) and 29 ALU instructions, 330 cycles of
+// an SM sub-partition per warp; 483 with a chain of low and a chain of high
+// halves per row (162 multiply-adds, 139 ALU).  A square takes 235 (308).
+// Inlined: at 113 and 107 instructions the walks' loops stay small enough for
+// the instruction caches.  Measured on B200 against one out-of-line body each:
+// grouped walk at G = 1024 5.11 G keys/s (5.07), at G = 64 4.53 (4.40), x-only
+// walk at B = 64 3.70 (3.54), pool 5.12 (5.10).  Before the aligned pairs:
+// 4.75, 4.03, 3.02 and 4.75, out of line.
+__device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) {
     fe o;
     fe_mul_ptx(o, a, b);
     return o;
 }
 
-static __device__ __noinline__ fe fe_sqr(const fe& a) {
+__device__ __forceinline__ fe fe_sqr(const fe& a) {
     fe o;
     fe_sqr_ptx(o, a);
     return o;

@@ -110,7 +110,7 @@ __device__ __forceinline__ void to_affine(const fe& X, const fe& Y, const fe& Z,
 
 // The table: thread i computes i Q (i = 1..M) and thread 0 computes J = 2M Q,
 // affine and canonical, into tu / tv ([M + 1] each).
-static __global__ void group_table_kernel(fe* tu, fe* tv, uint32_t m, fe q, fe vq) {
+static __global__ void __launch_bounds__(32) group_table_kernel(fe* tu, fe* tv, uint32_t m, fe q, fe vq) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > m) return;
     uint32_t s[8] = {i == 0 ? 2 * m : i, 0, 0, 0, 0, 0, 0, 0};

@@ -357,7 +357,7 @@ int build_group_table(lxmfv_handle* h) {
     cudaError_t e = cudaMalloc(&du, sizeof(fe) * (m + 1));
     if (e == cudaSuccess) e = cudaMalloc(&dv, sizeof(fe) * (m + 1));
     if (e == cudaSuccess) {
-        lxk::group_table_kernel<<<1, ((m + 1 + 31) / 32) * 32, 0, h->stream>>>(du, dv, m, u8b(), v8b());
+        lxk::group_table_kernel<<<(m + 1 + 31) / 32, 32, 0, h->stream>>>(du, dv, m, u8b(), v8b());
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->tu, du, sizeof(fe) * (m + 1), cudaMemcpyDeviceToHost, h->stream);

@@ -426,7 +426,7 @@ static int pool_open_body(const lxmfv_pool_options* opts, lxmfv_pool** out) {
     e = cudaMalloc(&du, sizeof(fe) * (p->m + 1));
     if (e == cudaSuccess) e = cudaMalloc(&dv, sizeof(fe) * (p->m + 1));
     if (e == cudaSuccess) {
-        lxk::group_table_kernel<<<1, ((p->m + 1 + 31) / 32) * 32, 0, p->stream>>>(du, dv, p->m, pool_u8b(),
+        lxk::group_table_kernel<<<(p->m + 1 + 31) / 32, 32, 0, p->stream>>>(du, dv, p->m, pool_u8b(),
                                                                                   pool_v8b());
         e = cudaGetLastError();
     }
