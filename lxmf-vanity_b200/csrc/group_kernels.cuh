@@ -44,6 +44,8 @@ struct GroupArgs {
     uint64_t* ns;     // [lanes]: walk index of the first key of the lane's next group (centre - M)
     uint32_t lanes;
     uint32_t iters;   // groups per lane in this launch
+    uint32_t parts;   // warps per 32 lanes (group_parts_kernel)
+    uint32_t* done;   // [lanes / 32]: warps that have finished their part; zero between launches
     EmitArgs em;
     GroupTable<M> t;
 };
@@ -70,6 +72,8 @@ struct GroupArgsConst {
     uint64_t* ns;
     uint32_t lanes;
     uint32_t iters;
+    uint32_t parts;
+    uint32_t* done;
     EmitArgs em;
 };
 template <int M>
@@ -173,18 +177,21 @@ static __global__ void __launch_bounds__(128) group_init_kernel(uint32_t* state,
 // phase of the walk, so that they share the instruction cache's working set
 // (one phase's code instead of all of it); every thread of the block must
 // then call this with the same `groups`.
+// lo, hi: the part of each group to walk, the keys c +- i with lo < i <= hi
+// (and the centre where lo is 0); 0 and M: all of it.  Every part steps to
+// the next centre by itself.
 template <int M, bool SYNC, class Table, class Emit>
 __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_t groups, const Table& t,
-                                            const Emit& emit) {
+                                            const Emit& emit, const int lo = 0, const int hi = M) {
     fe pre[M + 1];
     fe cA = fe_zero();
     cA.v[0] = LXK_A;
 #pragma unroll 1
     for (uint32_t it = 0; it < groups; ++it) {
-        // Denominators e_0 = u_J - u_C, e_i = u_{T_i} - u_C; pre[i] = e_0 ... e_{i-1}.
+        // Denominators e_0 = u_J - u_C, e_i = u_{T_i} - u_C; pre[i] = e_0 e_{lo+1} ... e_{i-1}.
         fe acc = fe_sub(t.u[0], uc);
 #pragma unroll 1
-        for (int i = 1; i <= M; ++i) {
+        for (int i = lo + 1; i <= hi; ++i) {
             pre[i] = acc;
             acc = fe_mul(acc, fe_sub(t.u[i], uc));
         }
@@ -193,7 +200,8 @@ __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_
         const fe s0 = fe_add(uc, cA);
         fe vnext = vc;
 #pragma unroll 1
-        for (int i = M; i >= 0; --i) {
+        for (int k = hi; k >= lo; --k) {
+            const int i = k > lo ? k : 0;  // last, the step to the next centre
             const fe tu = t.u[i], tv = t.v[i];
             fe invi = inv;  // 1 / e_i
             if (i > 0) {
@@ -214,8 +222,8 @@ __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_
 #pragma unroll 1
             for (int side = 0; side < 2; ++side) {
                 // side 0: key c + i (only 0 < i < M: c + M is the next group's);
-                // side 1: key c - i (i = 0: the centre).
-                if (side == 1 || (i > 0 && i < M)) {
+                // side 1: key c - i (i = 0: the centre, walked by the part that starts at 0).
+                if (side == 1 ? (i > 0 || lo == 0) : (i > 0 && i < M)) {
                     const fe u = fe_canon(side ? um : up);
                     emit(u, side ? c - (uint64_t)i : c + (uint64_t)i);
                 }
@@ -228,6 +236,59 @@ __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_
         n += 2 * M;
         if (SYNC) __syncthreads();
     }
+}
+
+// ---- Parts: each group split over several warps.
+//
+// A lane's groups are a serial chain, so a walk of few lanes leaves most of
+// the device idle, and one whose lanes are no multiple of a wave leaves its
+// last wave nearly empty.  The parts of a group are independent: 32 lanes are
+// walked by S warps, warp j the keys c +- i with floor(j M/S) < i <=
+// floor((j+1) M/S), each with its own batch inversion and its own step to the next centre.  Every
+// key, hash and hit is the one that a single warp finds.
+constexpr int kPartsWarps = 16;  // warps per block (512 threads, one block per SM)
+
+// S for `chunks` chunks of 32 lanes on `sms` SMs: the one with the smallest
+// predicted time, (ceil(M/S) + 4.1) x (full rounds of 16 warps per SM + the
+// last round's share).  Measured on B200: an inversion takes as long as
+// 4.1 pairs of keys at any occupancy, and a round of 1, 2, 3 or 4 warps per
+// SM sub-partition takes 10.2, 16.7, 23.9 or 31.1 us per pair (a lone warp
+// issues at three quarters of the full rate).  So few lanes split until
+// every sub-partition has a warp and the inversions (42 us at least) weigh as
+// much as the keys; full waves stay whole.
+inline uint32_t group_parts(uint64_t chunks, uint32_t m, uint32_t sms) {
+    static const uint32_t kRound[5] = {0, 21, 34, 49, 64};
+    const uint64_t slots = (uint64_t)sms * kPartsWarps;
+    uint32_t best = 1;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t s = 1; s <= m; s++) {
+        const uint64_t units = chunks * s, rest = units % slots;
+        const uint64_t rounds = units / slots * kRound[4] + kRound[(rest + 4 * sms - 1) / (4 * sms)];
+        const uint64_t cost = (10 * ((m + s - 1) / s) + 41) * rounds;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = s;
+        }
+    }
+    return best;
+}
+
+// Part j's first i, exclusive, and the next part's.
+__device__ __forceinline__ int part_begin(uint32_t m, uint32_t j, uint32_t parts) { return (int)(j * m / parts); }
+
+// A warp has walked its part of a chunk.  True for the last of the S
+// warps to come here, the one that stores the chunk's new state: by then the
+// others have read the old one.
+__device__ __forceinline__ bool part_done(uint32_t* done, uint32_t parts) {
+    if (parts == 1) return true;
+    uint32_t before = 0;
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence();
+        before = atomicAdd(done, 1u);
+        if (before == parts - 1) *done = 0;  // for the next launch
+    }
+    return __shfl_sync(0xffffffffu, before, 0) == parts - 1;
 }
 
 // The plain search's emission: one prefix for every lane of the launch.
@@ -260,6 +321,39 @@ static __global__ void __launch_bounds__(BLOCK, MINB) group_walk_kernel(const __
         store_fe(a.state, 0, lane, a.lanes, uc);
         store_fe(a.state, 1, lane, a.lanes, vc);
         a.ns[lane] = n;
+    }
+}
+
+// The plain walk in parts: one block per SM, whose warps take units of (32
+// lanes, part) a grid apart, so that the units of a short last round spread
+// over all SMs and their sub-partitions.  Lanes past the last one walk a copy
+// of it.  At G = 1024 on B200, one group: 32 lanes 15.2 -> 0.08 ms, 2,048
+// lanes 15.2 -> 0.54 ms, 100,003 lanes 30.3 -> 20.5 ms (5.00 G keys/s; a whole
+// wave 5.11).
+template <int M, bool DUMP, class Args = GroupArgsFor<M>>
+static __global__ void __launch_bounds__(32 * kPartsWarps, 1) group_parts_kernel(const __grid_constant__ Args a) {
+    const uint32_t lid = threadIdx.x & 31;
+    const uint32_t chunks = (a.lanes + 31) / 32, parts = a.parts;
+    const uint64_t units = (uint64_t)chunks * parts;
+#pragma unroll 1
+    for (uint64_t unit = blockIdx.x + (uint64_t)gridDim.x * (threadIdx.x >> 5); unit < units;
+         unit += (uint64_t)gridDim.x * kPartsWarps) {
+        const uint32_t chunk = (uint32_t)(unit / parts);
+        const uint32_t j = (uint32_t)(unit - (uint64_t)chunk * parts);
+        const bool active = chunk * 32 + lid < a.lanes;
+        const uint32_t lane = active ? chunk * 32 + lid : a.lanes - 1;
+        fe uc = load_fe(a.state, 0, lane, a.lanes);
+        fe vc = load_fe(a.state, 1, lane, a.lanes);
+        const uint64_t key0 = a.ns[lane];
+        uint64_t n = key0;
+        const LaneEmit<DUMP> emit{a.em, lane, key0, active};
+        walk_groups<M, false>(uc, vc, n, a.iters, table_of(a), emit, part_begin(M, j, parts),
+                              part_begin(M, j + 1, parts));
+        if (part_done(a.done + chunk, parts) && active) {
+            store_fe(a.state, 0, lane, a.lanes, uc);
+            store_fe(a.state, 1, lane, a.lanes, vc);
+            a.ns[lane] = n;
+        }
     }
 }
 

@@ -38,6 +38,7 @@ struct lxmfv_handle {
     uint32_t* d_err = nullptr;  // set by a warp-specialised launch whose wait gave up
     uint32_t* d_state = nullptr;
     uint64_t* d_ns = nullptr;
+    uint32_t* d_done = nullptr;  // grouped walk in parts: finished warps per 32 lanes
     uint32_t* d_hit_count = nullptr;
     lxk::Hit* d_hits = nullptr;
     uint32_t hits_cap = 0;
@@ -196,6 +197,8 @@ void launch_group_ws(lxmfv_handle* h, const lxk::EmitArgs& em, uint32_t iters) {
         a.g.ns = h->d_ns;
         a.g.lanes = h->lanes;
         a.g.iters = iters;
+        a.g.parts = 1;
+        a.g.done = nullptr;
         a.g.em = em;
         if constexpr (M <= 256) {
             for (int i = 0; i <= M; i++) {
@@ -225,8 +228,19 @@ void launch_group(lxmfv_handle* h, const lxk::EmitArgs& em, uint32_t iters) {
             ga.t.v[i] = h->tv[i];
         }
     }
-    const unsigned grid = (h->lanes + h->block - 1) / h->block;
     typedef void (*fn_t)(lxk::GroupArgsFor<M>);
+    // Whole waves of lanes run in the handle's launch shape, other counts in
+    // parts (group_parts); the register-capped build is always its own shape.
+    const uint64_t chunks = (h->lanes + 31) / 32;
+    ga.parts = lxk::group_parts(chunks, M, (uint32_t)h->sms);
+    ga.done = h->d_done;
+    if (!h->low_regs && (ga.parts > 1 || h->lanes % ((uint32_t)h->sms * 32 * lxk::kPartsWarps) != 0)) {
+        const unsigned grid = (unsigned)std::min<uint64_t>(h->sms, chunks * ga.parts);
+        const fn_t fn = em.dump_lanes > 0 ? (fn_t)lxk::group_parts_kernel<M, true> : (fn_t)lxk::group_parts_kernel<M, false>;
+        fn<<<grid, 32 * lxk::kPartsWarps, 0, h->stream>>>(ga);
+        return;
+    }
+    const unsigned grid = (h->lanes + h->block - 1) / h->block;
     const fn_t fn = (fn_t)group_kernel_ptr<M>(h->block, h->sync, h->low_regs, em.dump_lanes > 0);
     fn<<<grid, h->block, 0, h->stream>>>(ga);
 }
@@ -464,6 +478,8 @@ int lxmfv_open(const lxmfv_options* opts, lxmfv_handle** out) {
     }
     CU(h, cudaMalloc(&h->d_state, (size_t)h->lanes * 32 * sizeof(uint32_t)));
     CU(h, cudaMalloc(&h->d_ns, (size_t)h->lanes * sizeof(uint64_t)));
+    CU(h, cudaMalloc(&h->d_done, (size_t)((h->lanes + 31) / 32) * sizeof(uint32_t)));
+    CU(h, cudaMemsetAsync(h->d_done, 0, (size_t)((h->lanes + 31) / 32) * sizeof(uint32_t), h->stream));
     CU(h, cudaMalloc(&h->d_hit_count, sizeof(uint32_t)));
     CU(h, cudaMemsetAsync(h->d_hit_count, 0, sizeof(uint32_t), h->stream));
     CU(h, cudaMemsetAsync(h->d_state, 0, (size_t)h->lanes * 32 * sizeof(uint32_t), h->stream));
@@ -671,6 +687,7 @@ void lxmfv_close(lxmfv_handle* h) {
         if (h->stream) cudaStreamSynchronize(h->stream);
         cudaFree(h->d_state);
         cudaFree(h->d_ns);
+        cudaFree(h->d_done);
         cudaFree(h->d_hit_count);
         cudaFree(h->d_hits);
         cudaFree(h->d_dump_u);

@@ -13,16 +13,15 @@
 //     searches does not diverge;
 //   - lane state as in the grouped walk (u_C, v_C word-major, walk index);
 //   - a search table (the hash chain's constants per search slot);
-//   - the work queue: the active chunks, in search order.  Each step, the
-//     persistent kernel's blocks (one per SM, 16 warps) take items of 16
-//     chunks from it with an atomic counter until it is empty, and walk every
-//     lane of an item `groups` groups, so every active lane advances by the
-//     same number of keys per step: a search's hits do not depend on what
-//     else is in the pool;
+//   - the work queue: the active chunks, in search order, and the number of
+//     parts their groups are split into (group_parts).  Each step, the warps
+//     of the persistent kernel (one block of 16 warps per SM) take units of
+//     (chunk, part) a grid apart and walk them `groups` groups, so every
+//     active lane advances by the same number of keys per step: a search's
+//     hits do not depend on what else is in the pool;
 //   - a hit queue of (search, lane within the search, walk index).
-// One step is a CUDA graph, captured once per `groups`: reset the work
-// counter, run the persistent kernel, copy the hit count and hits to pinned
-// host memory.
+// One step is a CUDA graph, captured once per `groups`: run the persistent
+// kernel, copy the hit count and hits to pinned host memory.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,7 +47,7 @@ struct PoolHit {
     uint64_t n;
 };
 
-constexpr int kPoolWarps = 16;  // warps per block (512 threads)
+constexpr int kPoolWarps = kPartsWarps;  // warps per block (512 threads)
 
 // The pool's group table: in the parameters up to M = 256, in constant
 // memory (c_group_u / c_group_v, written at lxmfv_pool_open) at M = 512.
@@ -65,11 +64,11 @@ struct PoolArgs {
     uint64_t* ns;                  // [capacity]
     uint32_t capacity;
     const uint32_t* queue;         // active chunk ids
-    const uint32_t* n_queue;       // queue length (device scalar)
+    const uint32_t* n_queue;       // queue length and parts per chunk (2 device words)
     const uint32_t* chunk_search;  // [capacity / 32] search slot of each chunk
     const uint32_t* chunk_first;   // [capacity / 32] index in its search of the chunk's first lane
     const PoolSearch* searches;
-    uint32_t* head;                // work counter, zero at the start of a step
+    uint32_t* done;                // [capacity / 32]: warps that have finished their part; zero between steps
     uint32_t groups;               // groups per lane per step
     uint32_t* hit_count;
     PoolHit* hits;
@@ -85,14 +84,13 @@ struct PoolEmit {
     uint32_t max_hits;
     uint32_t search;
     uint32_t lane_in_search;
-    bool active;
     uint32_t one;  // from the kernel parameters
     __device__ __forceinline__ void operator()(const fe& u, uint64_t key) const {
         uint32_t d[4];
         lxsha::dest_hash_one(u.v, ac.ed, ac, one, d);
         const bool match = ((d[0] & ac.mask[0]) == ac.want[0]) & ((d[1] & ac.mask[1]) == ac.want[1]) &
                            ((d[2] & ac.mask[2]) == ac.want[2]) & ((d[3] & ac.mask[3]) == ac.want[3]);
-        if (active && match) {
+        if (match) {
             const uint32_t slot = atomicAdd(hit_count, 1u);
             if (slot < max_hits) {
                 hits[slot].search = search;
@@ -103,23 +101,25 @@ struct PoolEmit {
     }
 };
 
+// No barrier: the warps of a block start together and do equal work, so they
+// stay in one phase of the walk by themselves.  In items of 16 chunks per block
+// with a phase barrier, 636 chunks kept 40 of 148 SMs busy for 16.3 ms per group
+// of 1024; in parts, as units of a warp, they take 4.6 ms.  The full pool (9,472
+// chunks, one part) walks 5.08 G keys/s, 5.12 in items of 16.
 template <int M>
 static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(const __grid_constant__ PoolArgs<M> a) {
-    __shared__ uint32_t s_item;
     __shared__ lxsha::AddrConsts s_ac[kPoolWarps];
     const uint32_t warp = threadIdx.x >> 5, lid = threadIdx.x & 31;
-    const uint32_t nq = *a.n_queue;
-    const uint32_t n_items = (nq + kPoolWarps - 1) / kPoolWarps;
-    for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(a.head, 1u);
-        __syncthreads();
-        const uint32_t item = s_item;
-        if (item >= n_items) break;  // the same for every thread of the block
-        const uint32_t qi = item * kPoolWarps + warp;
-        const bool active = qi < nq;  // a short last item: spare warps walk a copy and write nothing
-        const uint32_t chunk = a.queue[active ? qi : nq - 1];
+    const uint32_t parts = a.n_queue[1];
+    const uint64_t units = (uint64_t)a.n_queue[0] * parts;
+#pragma unroll 1
+    for (uint64_t unit = blockIdx.x + (uint64_t)gridDim.x * warp; unit < units; unit += (uint64_t)gridDim.x * kPoolWarps) {
+        const uint32_t qi = (uint32_t)(unit / parts);
+        const uint32_t j = (uint32_t)(unit - (uint64_t)qi * parts);
+        const uint32_t chunk = a.queue[qi];
         const uint32_t search = a.chunk_search[chunk];
         constexpr int kWords = sizeof(lxsha::AddrConsts) / 4;
+        __syncwarp();  // the last unit's reads of s_ac are done
         if (lid < kWords)
             reinterpret_cast<uint32_t*>(&s_ac[warp])[lid] = reinterpret_cast<const uint32_t*>(&a.searches[search].ac)[lid];
         __syncwarp();
@@ -127,14 +127,14 @@ static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(co
         fe uc = load_fe(a.state, 0, lane, a.capacity);
         fe vc = load_fe(a.state, 1, lane, a.capacity);
         uint64_t n = a.ns[lane];
-        const PoolEmit emit{s_ac[warp], a.hit_count, a.hits, a.max_hits, search, a.chunk_first[chunk] + lid, active, a.one};
-        walk_groups<M, true>(uc, vc, n, a.groups, pool_table(a.t), emit);
-        if (active) {
+        const PoolEmit emit{s_ac[warp], a.hit_count, a.hits, a.max_hits, search, a.chunk_first[chunk] + lid, a.one};
+        walk_groups<M, false>(uc, vc, n, a.groups, pool_table(a.t), emit, part_begin(M, j, parts),
+                              part_begin(M, j + 1, parts));
+        if (part_done(a.done + chunk, parts)) {
             store_fe(a.state, 0, lane, a.capacity, uc);
             store_fe(a.state, 1, lane, a.capacity, vc);
             a.ns[lane] = n;
         }
-        __syncthreads();  // s_item and s_ac are rewritten next
     }
 }
 
@@ -177,7 +177,7 @@ struct lxmfv_pool {
     uint64_t* d_ns = nullptr;
     uint32_t *d_queue = nullptr, *d_nq = nullptr, *d_chunk_search = nullptr, *d_chunk_first = nullptr;
     lxk::PoolSearch* d_searches = nullptr;
-    uint32_t* d_head = nullptr;
+    uint32_t* d_done = nullptr;
     uint32_t* d_hit_count = nullptr;
     lxk::PoolHit* d_hits = nullptr;
     uint32_t* d_scalars = nullptr;  // staging for a submission's scalars
@@ -263,7 +263,7 @@ void launch_pool(lxmfv_pool* p, uint32_t groups) {
     a.chunk_search = p->d_chunk_search;
     a.chunk_first = p->d_chunk_first;
     a.searches = p->d_searches;
-    a.head = p->d_head;
+    a.done = p->d_done;
     a.groups = groups;
     a.hit_count = p->d_hit_count;
     a.hits = p->d_hits;
@@ -294,12 +294,13 @@ int rebuild_queue(lxmfv_pool* p) {
     for (const auto& s : p->searches)
         if (s.active) q.insert(q.end(), s.chunks.begin(), s.chunks.end());
     const uint32_t nq = (uint32_t)q.size();
+    const uint32_t head[2] = {nq, lxk::group_parts(nq, p->m, (uint32_t)p->sms)};
     if (nq) PCU(p, cudaMemcpyAsync(p->d_queue, q.data(), sizeof(uint32_t) * nq, cudaMemcpyHostToDevice, p->stream));
     PCU(p, cudaMemcpyAsync(p->d_chunk_search, p->h_chunk_search.data(), sizeof(uint32_t) * p->chunks,
                            cudaMemcpyHostToDevice, p->stream));
     PCU(p, cudaMemcpyAsync(p->d_chunk_first, p->h_chunk_first.data(), sizeof(uint32_t) * p->chunks,
                            cudaMemcpyHostToDevice, p->stream));
-    PCU(p, cudaMemcpyAsync(p->d_nq, &nq, sizeof nq, cudaMemcpyHostToDevice, p->stream));
+    PCU(p, cudaMemcpyAsync(p->d_nq, head, sizeof head, cudaMemcpyHostToDevice, p->stream));
     // The copies above read host memory that is gone after return: wait for them.
     PCU(p, cudaStreamSynchronize(p->stream));
     p->queue_dirty = false;
@@ -316,7 +317,6 @@ int capture_step(lxmfv_pool* p, uint32_t groups) {
         p->graph = nullptr;
     }
     PCU(p, cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(p->d_head, 0, sizeof(uint32_t), p->stream);
     launch_pool_any(p, groups);
     cudaMemcpyAsync(p->h_hit_count, p->d_hit_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, p->stream);
     cudaMemcpyAsync(p->h_hits, p->d_hits, sizeof(lxk::PoolHit) * p->max_hits, cudaMemcpyDeviceToHost, p->stream);
@@ -399,11 +399,11 @@ static int pool_open_body(const lxmfv_pool_options* opts, lxmfv_pool** out) {
     PCU(p, cudaMalloc(&p->d_state, (size_t)p->capacity * 16 * sizeof(uint32_t)));
     PCU(p, cudaMalloc(&p->d_ns, (size_t)p->capacity * sizeof(uint64_t)));
     PCU(p, cudaMalloc(&p->d_queue, (size_t)p->chunks * sizeof(uint32_t)));
-    PCU(p, cudaMalloc(&p->d_nq, sizeof(uint32_t)));
+    PCU(p, cudaMalloc(&p->d_nq, 2 * sizeof(uint32_t)));
     PCU(p, cudaMalloc(&p->d_chunk_search, (size_t)p->chunks * sizeof(uint32_t)));
     PCU(p, cudaMalloc(&p->d_chunk_first, (size_t)p->chunks * sizeof(uint32_t)));
     PCU(p, cudaMalloc(&p->d_searches, (size_t)p->max_searches * sizeof(lxk::PoolSearch)));
-    PCU(p, cudaMalloc(&p->d_head, sizeof(uint32_t)));
+    PCU(p, cudaMalloc(&p->d_done, (size_t)p->chunks * sizeof(uint32_t)));
     PCU(p, cudaMalloc(&p->d_hit_count, sizeof(uint32_t)));
     PCU(p, cudaMalloc(&p->d_hits, (size_t)p->max_hits * sizeof(lxk::PoolHit)));
     PCU(p, cudaMalloc(&p->d_scalars, (size_t)p->capacity * 32));
@@ -412,7 +412,8 @@ static int pool_open_body(const lxmfv_pool_options* opts, lxmfv_pool** out) {
     PCU(p, cudaMallocHost(&p->h_hits, (size_t)p->max_hits * sizeof(lxk::PoolHit)));
     *p->h_hit_count = 0;
     PCU(p, cudaMemsetAsync(p->d_hit_count, 0, sizeof(uint32_t), p->stream));
-    PCU(p, cudaMemsetAsync(p->d_nq, 0, sizeof(uint32_t), p->stream));
+    PCU(p, cudaMemsetAsync(p->d_nq, 0, 2 * sizeof(uint32_t), p->stream));
+    PCU(p, cudaMemsetAsync(p->d_done, 0, (size_t)p->chunks * sizeof(uint32_t), p->stream));
     PCU(p, cudaMemsetAsync(p->d_chunk_search, 0, (size_t)p->chunks * sizeof(uint32_t), p->stream));
     p->chunk_owner.assign(p->chunks, -1);
     p->h_chunk_search.assign(p->chunks, 0);
@@ -738,7 +739,7 @@ void lxmfv_pool_close(lxmfv_pool* p) {
         cudaFree(p->d_chunk_search);
         cudaFree(p->d_chunk_first);
         cudaFree(p->d_searches);
-        cudaFree(p->d_head);
+        cudaFree(p->d_done);
         cudaFree(p->d_hit_count);
         cudaFree(p->d_hits);
         cudaFree(p->d_scalars);

@@ -417,3 +417,47 @@ def test_self_test_shape(lx):
         pfx = lx.prefix_parse("b0")
         for t, k in hits:
             assert lx.prefix_matches(pfx, lx.address_of_identity(lx.step_scalar(bytes(scal[t]), k) + seed))
+
+
+@pytest.mark.parametrize("lanes,batch", [(1, 32), (1, 1024), (31, 64), (33, 1024), (1000, 256), (2400, 512), (4097, 1024)])
+def test_groups_in_parts_match_the_oracle(lx, oracle, lanes, batch):
+    """Lanes that are no whole wave are walked in parts, several warps per
+    chunk: part sizes that divide the group and that do not (1 pair per part
+    for one lane, 47 or 48 for 4,097 at G = 1024), a partial last chunk, and a
+    second launch that starts from the state the last part stored."""
+    with lx.Backend(device=0, lanes=lanes, batch=batch) as b:
+        setup = lx.seeded_setup(5151 + lanes, lanes)
+        b.init_from_scalars(setup.scalars)
+        look = sorted({0, lanes // 2, lanes - 1})
+        for launch in range(2):
+            args = lx.make_launch_args(2, setup.ed_pub, lx.prefix_parse("b0"), max_hits=1 << 16, dump_threads=lanes,
+                                       dump_keys=2 * batch)
+            hits, dump, addr, n = b.launch(args, want_dump=True, want_dump_addr=True)
+            assert n == len(hits)
+            keys = _keys_of(dump, lanes, 2 * batch)
+            hashes = _hashes_of(addr, lanes, 2 * batch)
+            for t in look:
+                walked = oracle.walk_keys(bytes(setup.scalars[t]), 4 * batch)[2 * batch * launch:2 * batch * (launch + 1)]
+                assert (keys[t] == walked).all(), (t, launch)
+            # Every hit, from the dumped hashes (which every key's own hash fills).
+            found = np.argwhere(hashes[:, :, 0] == 0xB0)
+            assert set(hits) == {(int(t), int(i) + 2 * batch * launch) for t, i in found}
+
+
+@pytest.mark.parametrize("block,flags,batch", [(128, 0, 32), (256, 0, 64), (256, 1, 128), (512, 0, 64), (512, 1, 1024)])
+def test_whole_waves_agree_with_the_x_only_walk(lx, block, flags, batch):
+    """A whole wave of lanes runs in the handle's launch shape."""
+    lanes = 148 * 512
+    setup = lx.seeded_setup(6262, lanes)
+    got = []
+    for walk, g, shape in ((lx.WALK_GROUP, batch, (block, flags)), (lx.WALK_XADD, 32, (0, 0))):
+        with lx.Backend(device=0, lanes=lanes, batch=g, block=shape[0], flags=shape[1], walk=walk) as b:
+            b.init_from_scalars(setup.scalars)
+            hits = set()
+            for _ in range(2):
+                args = lx.make_launch_args(max(32, batch) // g, setup.ed_pub, lx.prefix_parse("51d"), max_hits=1 << 16)
+                h, _, _, n = b.launch(args)
+                assert n == len(h)
+                hits.update(h)
+            got.append(hits)
+    assert got[0] == got[1] and len(got[0]) > 500
