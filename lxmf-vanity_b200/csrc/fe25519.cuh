@@ -15,6 +15,7 @@ struct __align__(16) fe {
 };
 
 #include "fe25519_ptx.cuh"
+#include "fe_divsteps.h"
 
 // Both are bound by the multiply-add pipe: a multiply is 72 aligned
 // 32 x 32 + 64 multiply-adds (half rate) and 29 ALU instructions, 330 cycles of
@@ -214,45 +215,11 @@ __device__ __forceinline__ fe fe_canon(const fe& a) {
     return o;
 }
 
-// The ref10 addition chain for z^(p-2) (254 squarings, 11 multiplications;
-// the chain of the reference's fe_invert, common.h:115-128), as a table that
-// a loop walks, so that its code holds one square and one multiply instead of
-// 265 inlined bodies.  After z2 = z^2, step s squares the running value
-// kSq[s] times and multiplies it by operand kOp[s]; kSave[s] names the slot
-// that keeps the result for a later step.
-// Operands: 0 z, 1 z2, 2 z9, 3 z11, 4 z^(2^10-1), 5 z^(2^50-1), 6 the step's
-// own input (z^(2^5-1), z^(2^10-1), ... doubling the run of ones).
-__device__ __constant__ uint8_t kInvSq[11] = {2, 0, 1, 5, 10, 20, 10, 50, 100, 50, 5};
-__device__ __constant__ uint8_t kInvOp[11] = {0, 1, 2, 6, 6, 6, 4, 6, 6, 5, 3};
-__device__ __constant__ uint8_t kInvSave[11] = {2, 3, 0, 4, 0, 0, 5, 0, 0, 0, 0};
-
-// z^(p-2).  0 maps to 0.  (static: each translation unit has its own copy.)
+// z^(p-2), canonical.  0 maps to 0.  (static: each translation unit has its own copy.)
 static __device__ __noinline__ fe fe_invert(fe z) {
-    fe z2 = fe_sqr(z);
-    fe z9 = z, z11 = z, z10 = z, z50 = z;
-    fe t = z2;
-#pragma unroll 1
-    for (int s = 0; s < 11; s++) {
-        const fe base = t;
-        const int n = kInvSq[s];
-#pragma unroll 1
-        for (int i = 0; i < n; i++) t = fe_sqr(t);
-        const int op = kInvOp[s];
-        fe m = base;
-        m = (op == 0) ? z : m;
-        m = (op == 1) ? z2 : m;
-        m = (op == 2) ? z9 : m;
-        m = (op == 3) ? z11 : m;
-        m = (op == 4) ? z10 : m;
-        m = (op == 5) ? z50 : m;
-        t = fe_mul(t, m);
-        const int sv = kInvSave[s];
-        z9 = (sv == 2) ? t : z9;
-        z11 = (sv == 3) ? t : z11;
-        z10 = (sv == 4) ? t : z10;
-        z50 = (sv == 5) ? t : z50;
-    }
-    return t;
+    fe o;
+    fed_invert(fe_canon(z).v, o.v);
+    return o;
 }
 
 // Conditional swap by mask (m all ones or all zeros), without branches.

@@ -13,7 +13,7 @@
 // C + T_i and C - T_i share the denominator u_T - u_C, so one batch inversion
 // (Montgomery's trick) over the M denominators and the step to the next
 // centre, C' = C + J with J = 2M Q, serves all 2M keys.  Per group:
-// (5M + 15) M + (2M + 254) S, i.e. about 2.6 M + 2.5 S per key at G = 128,
+// (5M + 4) M + (2M + 1) S and one inversion, about 2.5 M + 1 S per key,
 // against 8 M + 4 S for the x-only walk (G = B = 128).  The lane's local
 // buffer holds only the M prefix products (the denominators are recomputed
 // from the table on the way back).
@@ -249,13 +249,13 @@ __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_
 constexpr int kPartsWarps = 16;  // warps per block (512 threads, one block per SM)
 
 // S for `chunks` chunks of 32 lanes on `sms` SMs: the one with the smallest
-// predicted time, (ceil(M/S) + 4.1) x (full rounds of 16 warps per SM + the
-// last round's share).  Measured on B200: an inversion takes as long as
-// 4.1 pairs of keys at any occupancy, and a round of 1, 2, 3 or 4 warps per
-// SM sub-partition takes 10.2, 16.7, 23.9 or 31.1 us per pair (a lone warp
-// issues at three quarters of the full rate).  So few lanes split until
-// every sub-partition has a warp and the inversions (42 us at least) weigh as
-// much as the keys; full waves stay whole.
+// predicted time, (ceil(M/S) + 1.8) x (full rounds of 16 warps per SM + the
+// last round's share).  Measured on B200: an inversion with the step to
+// the next centre takes as long as 1.8 pairs of keys at any occupancy, and a
+// round of 1, 2, 3 or 4 warps per SM sub-partition takes 10.2, 16.7, 23.9 or
+// 31.1 us per pair (a lone warp issues at three quarters of the full rate).
+// So few lanes split until every sub-partition has a warp and the inversions
+// (16 us at least) weigh as much as the keys; full waves stay whole.
 inline uint32_t group_parts(uint64_t chunks, uint32_t m, uint32_t sms) {
     static const uint32_t kRound[5] = {0, 21, 34, 49, 64};
     const uint64_t slots = (uint64_t)sms * kPartsWarps;
@@ -264,7 +264,7 @@ inline uint32_t group_parts(uint64_t chunks, uint32_t m, uint32_t sms) {
     for (uint32_t s = 1; s <= m; s++) {
         const uint64_t units = chunks * s, rest = units % slots;
         const uint64_t rounds = units / slots * kRound[4] + kRound[(rest + 4 * sms - 1) / (4 * sms)];
-        const uint64_t cost = (10 * ((m + s - 1) / s) + 41) * rounds;
+        const uint64_t cost = (10 * ((m + s - 1) / s) + 18) * rounds;
         if (cost < best_cost) {
             best_cost = cost;
             best = s;

@@ -1,0 +1,40 @@
+"""The divsteps inversion, built for the CPU from the kernels' own header and
+checked against Python integers mod p = 2^255 - 19 (no GPU needed)."""
+import ctypes
+import os
+import random
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(__file__), "..", "lxmf-vanity_b200", "csrc")
+P = 2**255 - 19
+
+
+@pytest.fixture(scope="module")
+def invert(tmp_path_factory):
+    d = tmp_path_factory.mktemp("divsteps")
+    src = d / "inv.cpp"
+    src.write_text('#include "fe_divsteps.h"\nextern "C" void inv(const uint32_t* z, uint32_t* o) { fed_invert(z, o); }\n')
+    so = d / "inv.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-o", str(so), str(src)], check=True)
+    lib = ctypes.CDLL(str(so))
+
+    def call(z):
+        a = (ctypes.c_uint32 * 8)(*[(z >> (32 * i)) & 0xFFFFFFFF for i in range(8)])
+        o = (ctypes.c_uint32 * 8)()
+        lib.inv(a, o)
+        return sum(o[i] << (32 * i) for i in range(8))
+
+    return call
+
+
+@pytest.mark.parametrize("name", ["edges", "powers of two", "near p", "random"])
+def test_divsteps_inverse(invert, name):
+    rng = random.Random(17)
+    values = {"edges": [0, 1, 2, 18, 19, 20, P - 2, P - 1, (P - 1) // 2, (P + 1) // 2, 2**255 - 20],
+              "powers of two": [2**i for i in range(255)],
+              "near p": [P - 2**i for i in range(255)] + [2**255 - 2**i for i in range(5, 255)],
+              "random": [rng.randrange(P) for _ in range(5000)]}[name]
+    for z in values:
+        assert invert(z) == pow(z, P - 2, P), hex(z)  # canonical, and 0 for 0
