@@ -134,7 +134,7 @@ int lxmfv_init(lxmfv_handle* h, const uint32_t* u_prev_cur, size_t n_words);
 
 /* Sets every lane from its start scalar k (32 little-endian bytes per lane,
  * n_bytes = 32 * lanes; clamped, with room to step, as random_start_scalar
- * makes them, main.rs:157-171) by a Montgomery ladder on the GPU.  Replaces
+ * makes them, main.rs:157-171) by fixed-base multiplication on the GPU.  Replaces
  * first_public_keys (mod.rs:212-228), which runs two X25519 per lane on the
  * CPU, followed by Backend::init. */
 int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_bytes);

@@ -119,27 +119,9 @@ static __global__ void __launch_bounds__(32) group_table_kernel(fe* tu, fe* tv, 
     if (i > m) return;
     uint32_t s[8] = {i == 0 ? 2 * m : i, 0, 0, 0, 0, 0, 0, 0};
     fe x2, z2, x3, z3, X, Y, Z;
-    ladder(s, 32, q, x2, z2, x3, z3);
+    ladder(s, 11, q, x2, z2, x3, z3);  // 2M <= 1024
     recover_y(q, vq, x2, z2, x3, z3, X, Y, Z);
     to_affine(X, Y, Z, tu[i], tv[i]);
-}
-
-// Start from scalars: C = (k/8 + M) Q, the centre of the first group (walk
-// indices 0 .. 2M-1).
-static __global__ void __launch_bounds__(128) group_start_kernel(uint32_t* state, uint64_t* ns,
-                                                          const uint32_t* __restrict__ scalars, uint32_t lanes,
-                                                          uint32_t m, fe q, fe vq) {
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane >= lanes) return;
-    uint32_t s[8];
-    scalar_over_8(scalars, lane, (int)m, s);
-    fe x2, z2, x3, z3, X, Y, Z, u, v;
-    ladder(s, 253, q, x2, z2, x3, z3);
-    recover_y(q, vq, x2, z2, x3, z3, X, Y, Z);
-    to_affine(X, Y, Z, u, v);
-    store_fe(state, 0, lane, lanes, u);
-    store_fe(state, 1, lane, lanes, v);
-    ns[lane] = 0;
 }
 
 // Start from Backend::init's u(k-8), u(k): y of P = kB = (k/8) Q is recovered

@@ -16,6 +16,7 @@
 #include <string>
 
 #include "../../include/lxmfv.h"
+#include "comb_kernels.cuh"
 #include "group_kernels.cuh"
 #include "prim_kernels.cuh"
 #include "walk_kernels.cuh"
@@ -546,10 +547,11 @@ int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_by
     cudaError_t e = cudaMemcpyAsync(d, scalars, n_bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         if (h->walk == LXMFV_WALK_XADD) {
-            lxk::ladder_kernel<<<(h->lanes + 127) / 128, 128, 0, h->stream>>>(h->d_state, h->d_ns, d, h->lanes, u8b());
+            lxk::xonly_start_kernel<<<(h->lanes + 127) / 128, lxk::kCombThreads, 0, h->stream>>>(h->d_state, h->d_ns, d,
+                                                                                                 h->lanes);
         } else {
-            lxk::group_start_kernel<<<(h->lanes + 127) / 128, 128, 0, h->stream>>>(h->d_state, h->d_ns, d, h->lanes,
-                                                                                    h->batch / 2, u8b(), v8b());
+            lxk::group_start_kernel<<<(h->lanes + 127) / 128, lxk::kCombThreads, 0, h->stream>>>(h->d_state, h->d_ns, d,
+                                                                                                 h->lanes, h->batch / 2);
         }
         e = cudaGetLastError();
     }
@@ -573,7 +575,8 @@ int lxmfv_first_public_keys(lxmfv_handle* h, const uint8_t* scalars, size_t coun
     if (e == cudaSuccess) e = cudaMalloc(&dout, count * 64);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ds, scalars, count * 32, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
-        lxk::first_keys_kernel<<<(unsigned)((count + 127) / 128), 128, 0, h->stream>>>(dout, ds, (uint32_t)count, u8b());
+        lxk::first_keys_kernel<<<(unsigned)((count + 127) / 128), lxk::kCombThreads, 0, h->stream>>>(
+            reinterpret_cast<uint4*>(dout), ds, (uint32_t)count);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(u_prev_cur, dout, count * 64, cudaMemcpyDeviceToHost, h->stream);

@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/lxmfv.h"
+#include "comb_kernels.cuh"
 #include "group_kernels.cuh"
 
 namespace lxk {
@@ -138,20 +139,18 @@ static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(co
     }
 }
 
-// Start centres for `count` lanes of one search: lane i (a pool lane from
-// lane_map) from start scalar i, C = (k/8 + M) Q as in group_start_kernel.
-static __global__ void __launch_bounds__(128) pool_start_kernel(uint32_t* state, uint64_t* ns, uint32_t capacity,
+// Start centres for `count` lanes: lane i (a pool lane from lane_map) from
+// start scalar i, as in group_start_kernel.
+static __global__ void __launch_bounds__(kCombThreads) pool_start_kernel(uint32_t* state, uint64_t* ns, uint32_t capacity,
                                                                  const uint32_t* __restrict__ scalars,
                                                                  const uint32_t* __restrict__ lane_map, uint32_t count,
-                                                                 uint32_t m, fe q, fe vq) {
+                                                                 uint32_t m) {
+    __shared__ uint4 table[kCombVecs];
+    comb_stage(table);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    uint32_t s[8];
-    scalar_over_8(scalars, i, (int)m, s);
-    fe x2, z2, x3, z3, X, Y, Z, u, v;
-    ladder(s, 253, q, x2, z2, x3, z3);
-    recover_y(q, vq, x2, z2, x3, z3, X, Y, Z);
-    to_affine(X, Y, Z, u, v);
+    fe u, v;
+    start_centre(scalars, i, m, table, u, v);
     const uint32_t lane = lane_map[i];
     store_fe(state, 0, lane, capacity, u);
     store_fe(state, 1, lane, capacity, v);
@@ -510,8 +509,8 @@ static int pool_submit_body(lxmfv_pool* p, const lxmfv_search_desc* d, const uin
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(p->d_lane_map, lane_map.data(), sizeof(uint32_t) * d->lanes, cudaMemcpyHostToDevice, p->stream);
     if (e == cudaSuccess) {
-        lxk::pool_start_kernel<<<(d->lanes + 127) / 128, 128, 0, p->stream>>>(
-            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, d->lanes, p->m, pool_u8b(), pool_v8b());
+        lxk::pool_start_kernel<<<(d->lanes + 127) / 128, lxk::kCombThreads, 0, p->stream>>>(
+            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, d->lanes, p->m);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
@@ -611,9 +610,8 @@ static int pool_submit_many_body(lxmfv_pool* p, const lxmfv_search_desc* descs, 
         e = cudaMemcpyAsync(p->d_lane_map, lane_map.data(), sizeof(uint32_t) * lanes_total, cudaMemcpyHostToDevice,
                             p->stream);
     if (e == cudaSuccess) {
-        lxk::pool_start_kernel<<<(unsigned)((lanes_total + 127) / 128), 128, 0, p->stream>>>(
-            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, (uint32_t)lanes_total, p->m, pool_u8b(),
-            pool_v8b());
+        lxk::pool_start_kernel<<<(unsigned)((lanes_total + 127) / 128), lxk::kCombThreads, 0, p->stream>>>(
+            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, (uint32_t)lanes_total, p->m);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

@@ -232,42 +232,4 @@ __device__ __forceinline__ void scalar_over_8(const uint32_t* __restrict__ scala
     }
 }
 
-// x-only start: (P(-1), P(0)) = ((k-8)B, kB), left projective (replacing the
-// CPU start points of first_public_keys, mod.rs:212-228, for the walk).
-static __global__ void __launch_bounds__(128) ladder_kernel(uint32_t* state, uint64_t* ns, const uint32_t* __restrict__ scalars,
-                                                     uint32_t lanes, fe q) {
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane >= lanes) return;
-    uint32_t s[8];
-    scalar_over_8(scalars, lane, -1, s);
-    fe x2, z2, x3, z3;
-    ladder(s, 252, q, x2, z2, x3, z3);
-    store_fe(state, 0, lane, lanes, x2);
-    store_fe(state, 1, lane, lanes, z2);
-    store_fe(state, 2, lane, lanes, x3);
-    store_fe(state, 3, lane, lanes, z3);
-    ns[lane] = 0;
-}
-
-// first_public_keys (mod.rs:212-228) on the GPU: u(k-8) and u(k) as 16
-// canonical little-endian words per lane, the input of Backend::init.  One
-// inversion of Z2 * Z3 serves both coordinates.
-static __global__ void __launch_bounds__(128) first_keys_kernel(uint32_t* __restrict__ upc, const uint32_t* __restrict__ scalars,
-                                                         uint32_t lanes, fe q) {
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane >= lanes) return;
-    uint32_t s[8];
-    scalar_over_8(scalars, lane, -1, s);
-    fe x2, z2, x3, z3;
-    ladder(s, 252, q, x2, z2, x3, z3);
-    const fe inv = fe_invert(fe_mul(z2, z3));
-    const fe u_prev = fe_canon(fe_mul(x2, fe_mul(inv, z3)));
-    const fe u_cur = fe_canon(fe_mul(x3, fe_mul(inv, z2)));
-#pragma unroll
-    for (int w = 0; w < 8; w++) {
-        upc[(size_t)lane * 16 + w] = u_prev.v[w];
-        upc[(size_t)lane * 16 + 8 + w] = u_cur.v[w];
-    }
-}
-
 }  // namespace lxk

@@ -1,9 +1,11 @@
 """The divsteps inversion, built for the CPU from the kernels' own header and
-checked against Python integers mod p = 2^255 - 19 (no GPU needed)."""
+checked against Python integers mod p = 2^255 - 19, and the start points'
+table against its generator (no GPU needed)."""
 import ctypes
 import os
 import random
 import subprocess
+import sys
 
 import pytest
 
@@ -38,3 +40,8 @@ def test_divsteps_inverse(invert, name):
               "random": [rng.randrange(P) for _ in range(5000)]}[name]
     for z in values:
         assert invert(z) == pow(z, P - 2, P), hex(z)  # canonical, and 0 for 0
+
+
+def test_comb_table_is_current():
+    out = subprocess.run([sys.executable, os.path.join(CSRC, "gen_comb_table.py")], capture_output=True, text=True, check=True)
+    assert out.stdout == open(os.path.join(CSRC, "comb_table.cuh")).read()

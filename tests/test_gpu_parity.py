@@ -461,3 +461,36 @@ def test_whole_waves_agree_with_the_x_only_walk(lx, block, flags, batch):
                 hits.update(h)
             got.append(hits)
     assert got[0] == got[1] and len(got[0]) > 500
+
+
+def _edge_scalars():
+    """Scalars whose signed 4-bit digits reach their ends: k/8 of all 8s, 7s,
+    fs and 0s, the smallest and the largest start, one digit at a time."""
+    mids = [int("8" * 63, 16), int("7" * 63, 16), int("f" * 63, 16), 0, 1, int("80" * 31, 16), int("08" * 31, 16)]
+    ks = [(1 << 254) | ((m % (1 << 250)) << 3) for m in mids] + [(1 << 254) + 8, (1 << 255) - 16]
+    ks += [(1 << 254) | (0xf << (4 * i + 3)) % (1 << 254) for i in range(0, 62, 7)]
+    return [k & ~7 for k in ks if k != 1 << 254]
+
+
+@pytest.mark.parametrize("walk,count", [(0, 1), (0, 18), (0, 127), (1, 129), (1, 1)])
+def test_start_points_of_edge_scalars(lx, walk, count):
+    """The fixed-base multiplication at the ends of its digits and at counts
+    around a block, against OpenSSL's X25519: u(k - 8), u(k), and the first
+    keys of a walk started from the same scalars."""
+    edge = [k.to_bytes(32, "little") for k in _edge_scalars()]
+    rest, _ = lx.seeded_scalars(99, 0, 129)
+    scal = np.stack([np.frombuffer(b, np.uint8) for b in (edge + [bytes(r) for r in rest])[:count]])
+    with lx.Backend(device=0, lanes=count, batch=32, walk=walk) as b:
+        pair = b.first_public_keys(scal).view(np.uint8).reshape(count, 2, 32)
+        b.init_from_scalars(scal)
+        args = lx.make_launch_args(1, bytes(32), lx.prefix_parse("ffffffff"), dump_threads=count, dump_keys=32)
+        _, dump, _, _ = b.launch(args, want_dump=True)
+    keys = _keys_of(dump, count, 32)
+    for t in range(count):
+        k = bytes(scal[t])
+        assert bytes(pair[t, 0]) == lx.x25519_base(lx.previous_scalar(k)), t
+        assert bytes(pair[t, 1]) == lx.x25519_base(k), t
+        for n in (0, 1, 31):
+            if int.from_bytes(k, "little") + 8 * n >> 255:
+                continue  # past the last clamped scalar: the largest start has room for one step
+            assert bytes(keys[t, n]) == lx.x25519_base(lx.step_scalar(k, n)), (t, n)
