@@ -722,7 +722,10 @@ int lxmfv_fe_op(lxmfv_handle* h, int op, const uint32_t* a, const uint32_t* b, u
     if (e == cudaSuccess) {
         const int grid = h->sms * 8;
         if (op == 3) {
-            lxk::fe_batch_invert_kernel<<<grid, 128, 0, h->stream>>>(da, dout, count, group);
+            const uint64_t groups = (count + group - 1) / group;
+            const uint32_t t = lxk::invert_threads(groups, group, (uint32_t)h->sms);
+            lxk::batch_invert_kernel<<<(unsigned)((groups * t + lxk::kInvertThreads - 1) / lxk::kInvertThreads),
+                                       lxk::kInvertThreads, 0, h->stream>>>(da, dout, dout, count, group, t);
         } else {
             lxk::fe_op_kernel<<<grid, 256, 0, h->stream>>>(op, da, db, dout, count);
         }

@@ -38,7 +38,7 @@
 #include <mutex>
 
 #include "../../include/lxmfv.h"
-#include "fe25519.cuh"
+#include "batch_invert.cuh"
 
 namespace {
 
@@ -54,44 +54,6 @@ struct ScratchAddr {
 };
 ScratchAddr g_scratch[kMaxDevices];
 std::mutex g_setup_mutex;
-
-__device__ __forceinline__ fe load8_drop255(const uint32_t* p) {
-    const uint4* p4 = reinterpret_cast<const uint4*>(p);
-    const uint4 lo = p4[0], hi = p4[1];
-    fe r;
-    r.v[0] = lo.x; r.v[1] = lo.y; r.v[2] = lo.z; r.v[3] = lo.w;
-    r.v[4] = hi.x; r.v[5] = hi.y; r.v[6] = hi.z; r.v[7] = hi.w & 0x7fffffffu;
-    return r;
-}
-
-__device__ __forceinline__ void store8(uint32_t* p, const fe& x) {
-    uint4* p4 = reinterpret_cast<uint4*>(p);
-    p4[0] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-    p4[1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
-}
-
-// One group per thread: prefix products go to `scratch`, the inverses to
-// `out`.  `out` may be `a`: each element is read before its inverse is
-// stored, and a thread touches only its own group.
-__global__ void fe_batch_invert_scratch_kernel(const uint32_t* a, uint32_t* out, uint64_t count, uint32_t group,
-                                               fe* __restrict__ scratch) {
-    const uint64_t groups = (count + group - 1) / group;
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < groups; g += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t base = g * group;
-        const uint32_t len = (uint32_t)((count - base) < group ? (count - base) : group);
-        fe acc = fe_one();
-        for (uint32_t i = 0; i < len; i++) {
-            scratch[base + i] = acc;
-            acc = fe_mul(acc, load8_drop255(a + 8 * (base + i)));
-        }
-        fe inv = fe_invert(acc);
-        for (int i = (int)len - 1; i >= 0; i--) {
-            const fe ai = load8_drop255(a + 8 * (base + i));
-            store8(out + 8 * (base + i), fe_canon(fe_mul(inv, scratch[base + i])));
-            inv = fe_mul(inv, ai);
-        }
-    }
-}
 
 int say(char* err, size_t err_len, int code, const char* msg) {
     if (err && err_len) snprintf(err, err_len, "%s", msg);
@@ -151,6 +113,9 @@ extern "C" int lxmfv_fe_batch_invert_static(const uint32_t* d_a, uint32_t* d_out
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return say(err, err_len, LXMFV_ERR_CUDA, cudaGetErrorString(e));
     if (dev < 0 || dev >= kMaxDevices) return say(err, err_len, LXMFV_ERR_STATE, "device ordinal out of range");
+    int sms = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return say(err, err_len, LXMFV_ERR_CUDA, cudaGetErrorString(e));
     fe* scratch = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_setup_mutex);
@@ -170,9 +135,11 @@ extern "C" int lxmfv_fe_batch_invert_static(const uint32_t* d_a, uint32_t* d_out
             g_scratch[dev].addr = scratch;
         }
     }
-    const unsigned groups = (unsigned)((count + group - 1) / group);
-    const unsigned blocks = (groups + 127) / 128;
-    fe_batch_invert_scratch_kernel<<<blocks, 128, 0, (cudaStream_t)stream>>>(d_a, d_out, count, group, scratch);
+    const uint64_t groups = (count + group - 1) / group;
+    const uint32_t threads = lxk::invert_threads(groups, group, (uint32_t)sms);
+    const unsigned blocks = (unsigned)((groups * threads + lxk::kInvertThreads - 1) / lxk::kInvertThreads);
+    lxk::batch_invert_kernel<<<blocks, lxk::kInvertThreads, 0, (cudaStream_t)stream>>>(
+        d_a, d_out, reinterpret_cast<uint32_t*>(scratch), count, group, threads);
     e = cudaGetLastError();
     if (e != cudaSuccess) return say(err, err_len, LXMFV_ERR_CUDA, cudaGetErrorString(e));
     return LXMFV_OK;

@@ -3,37 +3,11 @@
 #pragma once
 #include <cstdint>
 
+#include "batch_invert.cuh"
 #include "fe25519.cuh"
 #include "sha256_lxmf.cuh"
 
 namespace lxk {
-
-// 8 words with bit 255 dropped, as the reference's fe_from_words reads them
-// (common.h:131-142).
-__device__ __forceinline__ fe load_words_drop255(const uint32_t* p) {
-    fe r;
-    const uint4* p4 = reinterpret_cast<const uint4*>(p);
-    const uint4 lo = p4[0], hi = p4[1];
-    r.v[0] = lo.x; r.v[1] = lo.y; r.v[2] = lo.z; r.v[3] = lo.w;
-    r.v[4] = hi.x; r.v[5] = hi.y; r.v[6] = hi.z; r.v[7] = hi.w & 0x7fffffffu;
-    return r;
-}
-
-// All 256 bits: an intermediate value of the 8-word representation.
-__device__ __forceinline__ fe load_words(const uint32_t* p) {
-    fe r;
-    const uint4* p4 = reinterpret_cast<const uint4*>(p);
-    const uint4 lo = p4[0], hi = p4[1];
-    r.v[0] = lo.x; r.v[1] = lo.y; r.v[2] = lo.z; r.v[3] = lo.w;
-    r.v[4] = hi.x; r.v[5] = hi.y; r.v[6] = hi.z; r.v[7] = hi.w;
-    return r;
-}
-
-__device__ __forceinline__ void store_words(uint32_t* p, const fe& x) {
-    uint4* p4 = reinterpret_cast<uint4*>(p);
-    p4[0] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-    p4[1] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
-}
 
 static __global__ void fe_op_kernel(int op, const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
                              uint32_t* __restrict__ out, uint64_t count) {
@@ -44,29 +18,6 @@ static __global__ void fe_op_kernel(int op, const uint32_t* __restrict__ a, cons
         else if (op == 1) r = fe_sqr(x);
         else r = fe_invert(x);
         store_words(out + 8 * i, fe_canon(r));
-    }
-}
-
-// Montgomery's trick over each group of `group` (<= 256) consecutive elements,
-// one group per thread; the structure of the walk's batch inversion.
-static __global__ void fe_batch_invert_kernel(const uint32_t* __restrict__ a, uint32_t* __restrict__ out, uint64_t count,
-                                       uint32_t group) {
-    const uint64_t groups = (count + group - 1) / group;
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < groups; g += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t base = g * group;
-        const uint32_t len = (uint32_t)((count - base) < group ? (count - base) : group);
-        // Prefix products go to the output buffer, then are overwritten.
-        fe acc = fe_one();
-        for (uint32_t i = 0; i < len; i++) {
-            store_words(out + 8 * (base + i), acc);
-            acc = fe_mul(acc, load_words_drop255(a + 8 * (base + i)));
-        }
-        fe inv = fe_invert(acc);
-        for (int i = (int)len - 1; i >= 0; i--) {
-            const fe pre = load_words(out + 8 * (base + i));
-            store_words(out + 8 * (base + i), fe_canon(fe_mul(inv, pre)));
-            inv = fe_mul(inv, load_words_drop255(a + 8 * (base + i)));
-        }
     }
 }
 

@@ -72,3 +72,26 @@ def test_static_scratch_rejects_bad_calls(lx):
     assert e.value.code == lx.ERR_ARG and "overlap" in str(e.value)
     torch.cuda.synchronize()
     assert int(d.abs().sum()) == 0  # nothing ran
+
+
+@pytest.mark.parametrize("count,group", [(1, 1), (6, 256), (40, 3), (1000, 33), (4099, 31), (9500, 2), (131072, 1),
+                                         (131071, 100), (131072, 256)])
+def test_groups_over_several_threads(lx, oracle, count, group):
+    """Groups split over 1 to 32 threads: runs of unequal length, groups
+    shorter than their threads, a short last group, more groups than threads
+    pay for; a zero zeroes its own group only."""
+    import torch
+
+    rng = np.random.default_rng(count + group)
+    torch.cuda.set_device(0)
+    a = rng.integers(0, 2**32, size=(count, 8), dtype=np.uint64).astype(np.uint32)
+    if count > 3 * group:
+        a[group] = 0
+        a[-1] = 0
+    d_a = torch.from_numpy(a.view(np.int32)).cuda()
+    d_out = torch.zeros_like(d_a)
+    torch.cuda.synchronize()
+    lx.fe_batch_invert_static(d_a.data_ptr(), d_out.data_ptr(), count, group)
+    torch.cuda.synchronize()
+    got = d_out.cpu().numpy().view(np.uint32)
+    assert (got == oracle.fe_batch_invert(a, group)).all()
