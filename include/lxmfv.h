@@ -75,9 +75,9 @@ typedef struct {
     int32_t device;       /* CUDA device ordinal */
     uint32_t lanes;       /* walker lanes (GPU threads); 0: one full wave of the device */
     uint32_t batch;       /* keys per inversion: XADD 16, 32, 64, 128; GROUP 32 .. 1024; 0: the fastest (GROUP 1024, XADD 128) */
-    uint32_t block;       /* threads per block: 128, 256 or 512; 0: 512 with LXMFV_FLAG_PHASE_SYNC.  The grouped walk
-                           * takes it for lanes in whole waves (512 per SM); other counts are walked in parts, several
-                           * warps per 32 lanes, in a shape of the library's own (not with REGCAP_80 or WARP_SPEC) */
+    uint32_t block;       /* threads per block: 128, 256 or 512; 0: 512 with LXMFV_FLAG_PHASE_SYNC.  It holds for
+                           * lanes in whole waves (512 per SM); other counts are walked in a shape of the library's own,
+                           * the grouped walk's in parts, several warps per 32 lanes (not with REGCAP_80 or WARP_SPEC) */
     uint32_t walk;        /* LXMFV_WALK_GROUP (0, default) or LXMFV_WALK_XADD */
     uint32_t flags;       /* LXMFV_FLAG_* */
     void* stream;         /* cudaStream_t to launch on; NULL: a stream of the handle's own */

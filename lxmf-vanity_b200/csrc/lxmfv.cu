@@ -182,10 +182,19 @@ const void* walk_kernel_ptr(uint32_t walk, uint32_t batch, uint32_t block, bool 
     return nullptr;
 }
 
+// Whole waves of lanes (512 per SM) run in the handle's launch shape; other
+// counts as units of a warp, spread over all SMs.
+bool whole_waves(const lxmfv_handle* h) { return h->lanes % ((uint32_t)h->sms * 512) == 0; }
+
 template <int B>
 void launch_xadd(lxmfv_handle* h, const lxk::WalkArgs& wa) {
-    const unsigned grid = (h->lanes + h->block - 1) / h->block;
     typedef void (*fn_t)(lxk::WalkArgs);
+    if (!whole_waves(h)) {
+        const fn_t fn = wa.em.dump_lanes > 0 ? (fn_t)lxk::walk_units_kernel<B, true> : (fn_t)lxk::walk_units_kernel<B, false>;
+        fn<<<std::min<unsigned>(h->sms, (h->lanes + 31) / 32), 32 * lxk::kUnitWarps, 0, h->stream>>>(wa);
+        return;
+    }
+    const unsigned grid = h->lanes / h->block;
     const fn_t fn = (fn_t)xadd_kernel_ptr<B>(h->block, h->sync, h->low_regs, wa.em.dump_lanes > 0);
     fn<<<grid, h->block, 0, h->stream>>>(wa);
 }
@@ -230,12 +239,12 @@ void launch_group(lxmfv_handle* h, const lxk::EmitArgs& em, uint32_t iters) {
         }
     }
     typedef void (*fn_t)(lxk::GroupArgsFor<M>);
-    // Whole waves of lanes run in the handle's launch shape, other counts in
-    // parts (group_parts); the register-capped build is always its own shape.
+    // Other counts than whole waves in parts; the register-capped build is
+    // always its own shape.
     const uint64_t chunks = (h->lanes + 31) / 32;
     ga.parts = lxk::group_parts(chunks, M, (uint32_t)h->sms);
     ga.done = h->d_done;
-    if (!h->low_regs && (ga.parts > 1 || h->lanes % ((uint32_t)h->sms * 32 * lxk::kPartsWarps) != 0)) {
+    if (!h->low_regs && (ga.parts > 1 || !whole_waves(h))) {
         const unsigned grid = (unsigned)std::min<uint64_t>(h->sms, chunks * ga.parts);
         const fn_t fn = em.dump_lanes > 0 ? (fn_t)lxk::group_parts_kernel<M, true> : (fn_t)lxk::group_parts_kernel<M, false>;
         fn<<<grid, 32 * lxk::kPartsWarps, 0, h->stream>>>(ga);

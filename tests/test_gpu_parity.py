@@ -494,3 +494,23 @@ def test_start_points_of_edge_scalars(lx, walk, count):
             if int.from_bytes(k, "little") + 8 * n >> 255:
                 continue  # past the last clamped scalar: the largest start has room for one step
             assert bytes(keys[t, n]) == lx.x25519_base(lx.step_scalar(k, n)), (t, n)
+
+
+@pytest.mark.parametrize("lanes,batch", [(1, 128), (33, 16), (4735, 64), (148 * 512 + 40, 32)])
+def test_xonly_units_agree_with_the_grouped_walk(lx, lanes, batch):
+    """x-only lanes that are no whole wave go by units of a warp: one lane, a
+    partial second chunk, a partial last chunk over all SMs, a second round."""
+    setup = lx.seeded_setup(7373 + lanes, lanes)
+    got = []
+    for walk, g in ((lx.WALK_XADD, batch), (lx.WALK_GROUP, 32)):
+        with lx.Backend(device=0, lanes=lanes, batch=g, walk=walk) as b:
+            b.init_from_scalars(setup.scalars)
+            hits = set()
+            for _ in range(2):
+                args = lx.make_launch_args(max(32, batch) // g, setup.ed_pub, lx.prefix_parse("3e" if lanes > 99 else "5"),
+                                           max_hits=1 << 16)
+                h, _, _, n = b.launch(args)
+                assert n == len(h)
+                hits.update(h)
+            got.append(hits)
+    assert got[0] == got[1] and got[0]
