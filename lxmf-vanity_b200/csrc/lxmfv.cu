@@ -40,9 +40,10 @@ struct lxmfv_handle {
     uint32_t* d_state = nullptr;
     uint64_t* d_ns = nullptr;
     uint32_t* d_done = nullptr;  // grouped walk in parts: finished warps per 32 lanes
-    uint32_t* d_hit_count = nullptr;
-    lxk::Hit* d_hits = nullptr;
+    uint8_t* d_hit_queue = nullptr;  // the hit count, padded to a hit, then hits_cap hits
     uint32_t hits_cap = 0;
+    uint8_t* d_work = nullptr;  // device copies of the array calls' host buffers, kept between calls
+    size_t work_cap = 0;
     uint32_t* d_dump_u = nullptr;
     uint32_t* d_dump_addr = nullptr;
     size_t dump_cap_keys = 0;
@@ -299,18 +300,65 @@ void fill_addr_consts(lxsha::AddrConsts& ac, const uint32_t ed[8], const uint32_
     }
 }
 
+uint32_t* hit_count(const lxmfv_handle* h) { return reinterpret_cast<uint32_t*>(h->d_hit_queue); }
+lxk::Hit* hit_slots(const lxmfv_handle* h) { return reinterpret_cast<lxk::Hit*>(h->d_hit_queue) + 1; }
+
+// Device memory for one array call (each waits for its work, so none overlap).
+// Up to kWorkKeep bytes stay with the handle: cudaMalloc and cudaFree cost 0.4
+// to 0.8 ms each on B200 and cudaFree waits for the device, against 0.5 ms for
+// the start points of a whole wave.  Larger buffers live for the call.
+constexpr size_t kWorkKeep = 128u << 20;
+constexpr uint64_t kMaxArray = 1ull << 33;  // elements; 32 bytes each are more than the device has
+struct Work {
+    uint8_t* base = nullptr;
+    bool owned = false;
+    size_t used = 0;
+    cudaError_t get(lxmfv_handle* h, size_t bytes) {
+        if (bytes > kWorkKeep) {
+            owned = true;
+            return cudaMalloc(&base, bytes);
+        }
+        if (bytes > h->work_cap) {
+            cudaFree(h->d_work);
+            h->d_work = nullptr;
+            h->work_cap = 0;
+            if (cudaError_t e = cudaMalloc(&h->d_work, bytes)) return e;
+            h->work_cap = bytes;
+        }
+        base = h->d_work;
+        return cudaSuccess;
+    }
+    static size_t size(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+    // The next `bytes` of the buffer.
+    uint32_t* take(size_t bytes) {
+        uint8_t* p = base + used;
+        used += size(bytes);
+        return reinterpret_cast<uint32_t*>(p);
+    }
+    ~Work() {
+        if (owned) cudaFree(base);
+    }
+};
+
 int ensure_hits(lxmfv_handle* h, uint32_t cap) {
     if (cap <= h->hits_cap) return LXMFV_OK;
     // Grow only between launches: every queued launch has finished here.
     CU(h, cudaStreamSynchronize(h->stream));
-    lxk::Hit* nh = nullptr;
-    CU(h, cudaMalloc(&nh, sizeof(lxk::Hit) * cap));
-    if (h->d_hits) {
-        CU(h, cudaMemcpyAsync(nh, h->d_hits, sizeof(lxk::Hit) * h->hits_cap, cudaMemcpyDeviceToDevice, h->stream));
-        CU(h, cudaStreamSynchronize(h->stream));
-        cudaFree(h->d_hits);
+    uint8_t* q = nullptr;
+    CU(h, cudaMalloc(&q, sizeof(lxk::Hit) * ((size_t)cap + 1)));
+    cudaError_t e;
+    if (h->d_hit_queue)
+        e = cudaMemcpyAsync(q, h->d_hit_queue, sizeof(lxk::Hit) * ((size_t)h->hits_cap + 1), cudaMemcpyDeviceToDevice,
+                            h->stream);
+    else
+        e = cudaMemsetAsync(q, 0, sizeof(lxk::Hit), h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) {
+        cudaFree(q);
+        return fail(h, LXMFV_ERR_CUDA, "hit queue: %s", cudaGetErrorString(e));
     }
-    h->d_hits = nh;
+    cudaFree(h->d_hit_queue);
+    h->d_hit_queue = q;
     h->hits_cap = cap;
     return LXMFV_OK;
 }
@@ -366,9 +414,9 @@ int check_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t count) {
         const uint8_t* k = scalars + 32 * t;
         if ((k[0] & 7) != 0 || (k[31] & 0xC0) != 0x40)
             return fail(h, LXMFV_ERR_ARG, "scalar %zu is not clamped (k mod 8 = 0, bit 254 set, bit 255 clear)", t);
-        bool low_all_clear = k[31] == 64;
-        for (int i = 0; i < 31; i++) low_all_clear = low_all_clear && k[i] == 0;
-        if (low_all_clear) return fail(h, LXMFV_ERR_ARG, "scalar %zu is 2^254: k - 8 would not be clamped", t);
+        static const uint8_t kLeast[32] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0,
+                                           0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 64};
+        if (k[31] == 64 && memcmp(k, kLeast, 32) == 0) return fail(h, LXMFV_ERR_ARG, "scalar %zu is 2^254: k - 8 would not be clamped", t);
     }
     return LXMFV_OK;
 }
@@ -490,8 +538,6 @@ int lxmfv_open(const lxmfv_options* opts, lxmfv_handle** out) {
     CU(h, cudaMalloc(&h->d_ns, (size_t)h->lanes * sizeof(uint64_t)));
     CU(h, cudaMalloc(&h->d_done, (size_t)((h->lanes + 31) / 32) * sizeof(uint32_t)));
     CU(h, cudaMemsetAsync(h->d_done, 0, (size_t)((h->lanes + 31) / 32) * sizeof(uint32_t), h->stream));
-    CU(h, cudaMalloc(&h->d_hit_count, sizeof(uint32_t)));
-    CU(h, cudaMemsetAsync(h->d_hit_count, 0, sizeof(uint32_t), h->stream));
     CU(h, cudaMemsetAsync(h->d_state, 0, (size_t)h->lanes * 32 * sizeof(uint32_t), h->stream));
     CU(h, cudaMemsetAsync(h->d_ns, 0, (size_t)h->lanes * sizeof(uint64_t), h->stream));
     if (int rc = ensure_hits(h, 4096)) return rc;
@@ -522,8 +568,9 @@ int lxmfv_init(lxmfv_handle* h, const uint32_t* u_prev_cur, size_t n_words) {
         return fail(h, LXMFV_ERR_ARG, "u_prev_cur has %zu words; %u lanes need %zu", n_words, h->lanes,
                     (size_t)h->lanes * 16);
     if (int rc = set_device(h)) return rc;
-    uint32_t* d = nullptr;
-    CU(h, cudaMalloc(&d, n_words * sizeof(uint32_t)));
+    Work w;
+    CU(h, w.get(h, n_words * sizeof(uint32_t)));
+    uint32_t* d = w.take(n_words * sizeof(uint32_t));
     cudaError_t e = cudaMemcpyAsync(d, u_prev_cur, n_words * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         if (h->walk == LXMFV_WALK_XADD) {
@@ -536,7 +583,6 @@ int lxmfv_init(lxmfv_handle* h, const uint32_t* u_prev_cur, size_t n_words) {
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(d);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "init: %s", cudaGetErrorString(e));
     h->initialised = true;
     h->err.clear();
@@ -551,8 +597,9 @@ int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_by
                     (size_t)h->lanes * 32);
     if (int rc = check_scalars(h, scalars, h->lanes)) return rc;
     if (int rc = set_device(h)) return rc;
-    uint32_t* d = nullptr;
-    CU(h, cudaMalloc(&d, n_bytes));
+    Work w;
+    CU(h, w.get(h, n_bytes));
+    uint32_t* d = w.take(n_bytes);
     cudaError_t e = cudaMemcpyAsync(d, scalars, n_bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         if (h->walk == LXMFV_WALK_XADD) {
@@ -565,7 +612,6 @@ int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_by
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(d);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "init_from_scalars: %s", cudaGetErrorString(e));
     h->initialised = true;
     h->err.clear();
@@ -579,10 +625,10 @@ int lxmfv_first_public_keys(lxmfv_handle* h, const uint8_t* scalars, size_t coun
     if (count > (1u << 30)) return fail(h, LXMFV_ERR_ARG, "count %zu too large", count);
     if (int rc = check_scalars(h, scalars, count)) return rc;
     if (int rc = set_device(h)) return rc;
-    uint32_t *ds = nullptr, *dout = nullptr;
-    cudaError_t e = cudaMalloc(&ds, count * 32);
-    if (e == cudaSuccess) e = cudaMalloc(&dout, count * 64);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ds, scalars, count * 32, cudaMemcpyHostToDevice, h->stream);
+    Work w;
+    CU(h, w.get(h, Work::size(count * 32) + count * 64));
+    uint32_t *ds = w.take(count * 32), *dout = w.take(count * 64);
+    cudaError_t e = cudaMemcpyAsync(ds, scalars, count * 32, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         lxk::first_keys_kernel<<<(unsigned)((count + 127) / 128), lxk::kCombThreads, 0, h->stream>>>(
             reinterpret_cast<uint4*>(dout), ds, (uint32_t)count);
@@ -590,8 +636,6 @@ int lxmfv_first_public_keys(lxmfv_handle* h, const uint8_t* scalars, size_t coun
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(u_prev_cur, dout, count * 64, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(ds);
-    cudaFree(dout);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "first_public_keys: %s", cudaGetErrorString(e));
     h->err.clear();
     return LXMFV_OK;
@@ -615,8 +659,8 @@ int lxmfv_launch_async(lxmfv_handle* h, const lxmfv_launch_args* args) {
     memset(&em, 0, sizeof em);
     fill_addr_consts(em.ac, args->ed, args->name_hash, args->want, args->mask);
     if (int rc = ensure_hits(h, std::max<uint32_t>(args->max_hits, 1))) return rc;
-    em.hit_count = h->d_hit_count;
-    em.hits = h->d_hits;
+    em.hit_count = hit_count(h);
+    em.hits = hit_slots(h);
     em.max_hits = args->max_hits;
     h->launch_max_hits = std::max(h->launch_max_hits, args->max_hits);
     if (args->dump_threads > 0) {
@@ -646,23 +690,30 @@ int lxmfv_collect(lxmfv_handle* h, lxmfv_hit* hits, uint32_t hits_cap, uint32_t*
                   uint32_t* dump_addr) {
     if (!h || !n_hits) return fail(h, LXMFV_ERR_ARG, "null argument");
     if (int rc = set_device(h)) return rc;
+    // The count and the first hits come in one copy; a search rarely has more.
+    constexpr uint32_t kFirst = 255;
+    lxk::Hit first[kFirst + 1];
+    const uint32_t have = std::min(kFirst, h->hits_cap);
+    CU(h, cudaMemcpyAsync(first, h->d_hit_queue, sizeof(lxk::Hit) * (have + 1), cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
-    uint32_t count = 0;
-    CU(h, cudaMemcpy(&count, h->d_hit_count, sizeof count, cudaMemcpyDeviceToHost));
+    uint32_t count;
+    memcpy(&count, first, sizeof count);
     const uint32_t stored = std::min(std::min(count, h->launch_max_hits), h->hits_cap);
     const uint32_t give = hits ? std::min(stored, hits_cap) : 0;
-    if (give > 0) CU(h, cudaMemcpy(hits, h->d_hits, sizeof(lxk::Hit) * give, cudaMemcpyDeviceToHost));
+    if (give > 0) memcpy(hits, first + 1, sizeof(lxk::Hit) * std::min(give, have));
+    if (give > have)
+        CU(h, cudaMemcpy(hits + have, hit_slots(h) + have, sizeof(lxk::Hit) * (give - have), cudaMemcpyDeviceToHost));
     const size_t dumped = (size_t)h->dump_lanes * h->dump_keys;
     if (dump && dumped) CU(h, cudaMemcpy(dump, h->d_dump_u, dumped * 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
     if (dump_addr && dumped)
         CU(h, cudaMemcpy(dump_addr, h->d_dump_addr, dumped * 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    CU(h, cudaMemsetAsync(h->d_hit_count, 0, sizeof(uint32_t), h->stream));
+    // Cleared in the stream's order, before any later launch of the handle.
+    CU(h, cudaMemsetAsync(h->d_hit_queue, 0, sizeof(uint32_t), h->stream));
     uint32_t gave_up = 0;
     if (h->d_err) {
         CU(h, cudaMemcpy(&gave_up, h->d_err, sizeof gave_up, cudaMemcpyDeviceToHost));
         CU(h, cudaMemsetAsync(h->d_err, 0, sizeof(uint32_t), h->stream));
     }
-    CU(h, cudaStreamSynchronize(h->stream));
     h->launch_max_hits = 0;
     if (gave_up) {
         // Some lanes stopped part-way: their state no longer matches their walk index.
@@ -700,8 +751,8 @@ void lxmfv_close(lxmfv_handle* h) {
         cudaFree(h->d_state);
         cudaFree(h->d_ns);
         cudaFree(h->d_done);
-        cudaFree(h->d_hit_count);
-        cudaFree(h->d_hits);
+        cudaFree(h->d_hit_queue);
+        cudaFree(h->d_work);
         cudaFree(h->d_dump_u);
         cudaFree(h->d_dump_addr);
         cudaFree(h->d_err);
@@ -720,13 +771,13 @@ int lxmfv_fe_op(lxmfv_handle* h, int op, const uint32_t* a, const uint32_t* b, u
     if (op < 0 || op > 3) return fail(h, LXMFV_ERR_ARG, "op %d: 0 mul, 1 square, 2 invert, 3 batch invert", op);
     if (op == 3 && (group < 1 || group > 256)) return fail(h, LXMFV_ERR_ARG, "group %u not in 1..256", group);
     if (count == 0) return LXMFV_OK;
+    if (count > kMaxArray) return fail(h, LXMFV_ERR_CUDA, "fe_op: out of memory");
     if (int rc = set_device(h)) return rc;
     const size_t bytes = count * 8 * sizeof(uint32_t);
-    uint32_t *da = nullptr, *db = nullptr, *dout = nullptr;
-    cudaError_t e = cudaMalloc(&da, bytes);
-    if (e == cudaSuccess && op == 0) e = cudaMalloc(&db, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&dout, bytes);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(da, a, bytes, cudaMemcpyHostToDevice, h->stream);
+    Work w;
+    CU(h, w.get(h, (op == 0 ? 3 : 2) * Work::size(bytes)));
+    uint32_t *da = w.take(bytes), *dout = w.take(bytes), *db = op == 0 ? w.take(bytes) : nullptr;
+    cudaError_t e = cudaMemcpyAsync(da, a, bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess && op == 0) e = cudaMemcpyAsync(db, b, bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         const int grid = h->sms * 8;
@@ -742,9 +793,6 @@ int lxmfv_fe_op(lxmfv_handle* h, int op, const uint32_t* a, const uint32_t* b, u
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, bytes, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(da);
-    cudaFree(db);
-    cudaFree(dout);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "fe_op: %s", cudaGetErrorString(e));
     return LXMFV_OK;
 }
@@ -753,24 +801,23 @@ int lxmfv_address_chain(lxmfv_handle* h, const uint8_t* pks, const uint8_t name_
                         uint64_t count) {
     if (!h || !pks || !name_hash || !out) return fail(h, LXMFV_ERR_ARG, "null argument");
     if (count == 0) return LXMFV_OK;
+    if (count > kMaxArray) return fail(h, LXMFV_ERR_CUDA, "address_chain: out of memory");
     if (int rc = set_device(h)) return rc;
     uint32_t nh[3] = {(uint32_t)name_hash[0] << 24 | (uint32_t)name_hash[1] << 16 | (uint32_t)name_hash[2] << 8 | name_hash[3],
                       (uint32_t)name_hash[4] << 24 | (uint32_t)name_hash[5] << 16 | (uint32_t)name_hash[6] << 8 | name_hash[7],
                       (uint32_t)name_hash[8] << 24 | (uint32_t)name_hash[9] << 16};
     lxsha::AddrConsts ac;
     fill_addr_consts(ac, nullptr, nh, nullptr, nullptr);
-    uint32_t *dpk = nullptr, *dout = nullptr;
-    cudaError_t e = cudaMalloc(&dpk, count * 64);
-    if (e == cudaSuccess) e = cudaMalloc(&dout, count * 16);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dpk, pks, count * 64, cudaMemcpyHostToDevice, h->stream);
+    Work w;
+    CU(h, w.get(h, Work::size(count * 64) + count * 16));
+    uint32_t *dpk = w.take(count * 64), *dout = w.take(count * 16);
+    cudaError_t e = cudaMemcpyAsync(dpk, pks, count * 64, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         lxk::address_chain_kernel<<<h->sms * 8, 256, 0, h->stream>>>(dpk, ac, dout, count);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, count * 16, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(dpk);
-    cudaFree(dout);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "address_chain: %s", cudaGetErrorString(e));
     return LXMFV_OK;
 }

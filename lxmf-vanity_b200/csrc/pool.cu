@@ -64,10 +64,8 @@ struct PoolArgs {
     uint32_t* state;               // [16][capacity]: u_C, v_C
     uint64_t* ns;                  // [capacity]
     uint32_t capacity;
-    const uint32_t* queue;         // active chunk ids
-    const uint32_t* n_queue;       // queue length and parts per chunk (2 device words)
-    const uint32_t* chunk_search;  // [capacity / 32] search slot of each chunk
-    const uint32_t* chunk_first;   // [capacity / 32] index in its search of the chunk's first lane
+    const uint4* queue;            // [0]: queue length, parts per chunk; then for each active chunk: chunk, search
+                                   // slot, index in the search of the chunk's first lane
     const PoolSearch* searches;
     uint32_t* done;                // [capacity / 32]: warps that have finished their part; zero between steps
     uint32_t groups;               // groups per lane per step
@@ -111,14 +109,15 @@ template <int M>
 static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(const __grid_constant__ PoolArgs<M> a) {
     __shared__ lxsha::AddrConsts s_ac[kPoolWarps];
     const uint32_t warp = threadIdx.x >> 5, lid = threadIdx.x & 31;
-    const uint32_t parts = a.n_queue[1];
-    const uint64_t units = (uint64_t)a.n_queue[0] * parts;
+    const uint4 head = a.queue[0];
+    const uint32_t parts = head.y;
+    const uint64_t units = (uint64_t)head.x * parts;
 #pragma unroll 1
     for (uint64_t unit = blockIdx.x + (uint64_t)gridDim.x * warp; unit < units; unit += (uint64_t)gridDim.x * kPoolWarps) {
         const uint32_t qi = (uint32_t)(unit / parts);
         const uint32_t j = (uint32_t)(unit - (uint64_t)qi * parts);
-        const uint32_t chunk = a.queue[qi];
-        const uint32_t search = a.chunk_search[chunk];
+        const uint4 entry = a.queue[1 + qi];
+        const uint32_t chunk = entry.x, search = entry.y;
         constexpr int kWords = sizeof(lxsha::AddrConsts) / 4;
         __syncwarp();  // the last unit's reads of s_ac are done
         if (lid < kWords)
@@ -128,7 +127,7 @@ static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(co
         fe uc = load_fe(a.state, 0, lane, a.capacity);
         fe vc = load_fe(a.state, 1, lane, a.capacity);
         uint64_t n = a.ns[lane];
-        const PoolEmit emit{s_ac[warp], a.hit_count, a.hits, a.max_hits, search, a.chunk_first[chunk] + lid, a.one};
+        const PoolEmit emit{s_ac[warp], a.hit_count, a.hits, a.max_hits, search, entry.z + lid, a.one};
         walk_groups<M, false>(uc, vc, n, a.groups, pool_table(a.t), emit, part_begin(M, j, parts),
                               part_begin(M, j + 1, parts));
         if (part_done(a.done + chunk, parts)) {
@@ -159,7 +158,14 @@ static __global__ void __launch_bounds__(kCombThreads) pool_start_kernel(uint32_
 
 }  // namespace lxk
 
+// Hits that a step's graph copies to the host with their count (a poll
+// fetches the others): 4 KB per step; all 65,536 slots took 20 us of it.
+constexpr uint32_t kPoolFirstHits = 255;
+
 struct lxmfv_pool {
+    uint32_t* hit_count() const { return reinterpret_cast<uint32_t*>(d_hit_queue); }
+    lxk::PoolHit* hit_slots() const { return reinterpret_cast<lxk::PoolHit*>(d_hit_queue) + 1; }
+    size_t first_bytes() const { return sizeof(lxk::PoolHit) * (1 + (size_t)std::min(kPoolFirstHits, max_hits)); }
     struct Search {
         bool active = false;
         uint32_t lanes = 0;
@@ -174,17 +180,15 @@ struct lxmfv_pool {
     uint32_t capacity = 0, chunks = 0, max_searches = 0, max_hits = 0;
     uint32_t* d_state = nullptr;
     uint64_t* d_ns = nullptr;
-    uint32_t *d_queue = nullptr, *d_nq = nullptr, *d_chunk_search = nullptr, *d_chunk_first = nullptr;
+    uint4* d_queue = nullptr;
     lxk::PoolSearch* d_searches = nullptr;
     uint32_t* d_done = nullptr;
-    uint32_t* d_hit_count = nullptr;
-    lxk::PoolHit* d_hits = nullptr;
+    uint8_t* d_hit_queue = nullptr;  // the hit count, padded to a hit, then max_hits hits
     uint32_t* d_scalars = nullptr;  // staging for a submission's scalars
     uint32_t* d_lane_map = nullptr;
-    uint32_t* h_hit_count = nullptr;  // pinned
-    lxk::PoolHit* h_hits = nullptr;   // pinned
+    uint8_t* h_hit_queue = nullptr;  // pinned: the count and the first kPoolFirstHits hits, copied by every step
     std::vector<int32_t> chunk_owner;  // search slot or -1
-    std::vector<uint32_t> h_chunk_search, h_chunk_first;  // mirrors of the device chunk tables
+    std::vector<uint4> h_queue;  // what rebuild_queue uploads
     std::vector<uint32_t> free_chunks;
     std::vector<Search> searches;
     bool queue_dirty = true;
@@ -258,14 +262,11 @@ void launch_pool(lxmfv_pool* p, uint32_t groups) {
     a.ns = p->d_ns;
     a.capacity = p->capacity;
     a.queue = p->d_queue;
-    a.n_queue = p->d_nq;
-    a.chunk_search = p->d_chunk_search;
-    a.chunk_first = p->d_chunk_first;
     a.searches = p->d_searches;
     a.done = p->d_done;
     a.groups = groups;
-    a.hit_count = p->d_hit_count;
-    a.hits = p->d_hits;
+    a.hit_count = p->hit_count();
+    a.hits = p->hit_slots();
     a.max_hits = p->max_hits;
     a.one = 1;
     if constexpr (M <= 256) {
@@ -287,21 +288,20 @@ void launch_pool_any(lxmfv_pool* p, uint32_t groups) {
     }
 }
 
+// The work queue, in one upload (from pageable memory: copied out before the
+// call returns, and ordered after the steps already on the stream).
 int rebuild_queue(lxmfv_pool* p) {
-    std::vector<uint32_t> q;
-    q.reserve(p->chunks);
-    for (const auto& s : p->searches)
-        if (s.active) q.insert(q.end(), s.chunks.begin(), s.chunks.end());
-    const uint32_t nq = (uint32_t)q.size();
-    const uint32_t head[2] = {nq, lxk::group_parts(nq, p->m, (uint32_t)p->sms)};
-    if (nq) PCU(p, cudaMemcpyAsync(p->d_queue, q.data(), sizeof(uint32_t) * nq, cudaMemcpyHostToDevice, p->stream));
-    PCU(p, cudaMemcpyAsync(p->d_chunk_search, p->h_chunk_search.data(), sizeof(uint32_t) * p->chunks,
-                           cudaMemcpyHostToDevice, p->stream));
-    PCU(p, cudaMemcpyAsync(p->d_chunk_first, p->h_chunk_first.data(), sizeof(uint32_t) * p->chunks,
-                           cudaMemcpyHostToDevice, p->stream));
-    PCU(p, cudaMemcpyAsync(p->d_nq, head, sizeof head, cudaMemcpyHostToDevice, p->stream));
-    // The copies above read host memory that is gone after return: wait for them.
-    PCU(p, cudaStreamSynchronize(p->stream));
+    auto& q = p->h_queue;
+    q.assign(1, make_uint4(0, 0, 0, 0));
+    for (uint32_t slot = 0; slot < p->max_searches; slot++) {
+        const auto& s = p->searches[slot];
+        if (s.active)
+            for (uint32_t i = 0; i < s.chunks.size(); i++) q.push_back(make_uint4(s.chunks[i], slot, 32 * i, 0));
+    }
+    const uint32_t nq = (uint32_t)q.size() - 1;
+    q[0].x = nq;
+    q[0].y = lxk::group_parts(nq, p->m, (uint32_t)p->sms);
+    PCU(p, cudaMemcpyAsync(p->d_queue, q.data(), sizeof(uint4) * q.size(), cudaMemcpyHostToDevice, p->stream));
     p->queue_dirty = false;
     return LXMFV_OK;
 }
@@ -317,8 +317,7 @@ int capture_step(lxmfv_pool* p, uint32_t groups) {
     }
     PCU(p, cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
     launch_pool_any(p, groups);
-    cudaMemcpyAsync(p->h_hit_count, p->d_hit_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, p->stream);
-    cudaMemcpyAsync(p->h_hits, p->d_hits, sizeof(lxk::PoolHit) * p->max_hits, cudaMemcpyDeviceToHost, p->stream);
+    cudaMemcpyAsync(p->h_hit_queue, p->d_hit_queue, p->first_bytes(), cudaMemcpyDeviceToHost, p->stream);
     PCU(p, cudaStreamEndCapture(p->stream, &p->graph));
     PCU(p, cudaGraphInstantiate(&p->graph_exec, p->graph, 0));
     p->graph_groups = groups;
@@ -397,26 +396,18 @@ static int pool_open_body(const lxmfv_pool_options* opts, lxmfv_pool** out) {
     PCU(p, cudaEventCreate(&p->ev1));
     PCU(p, cudaMalloc(&p->d_state, (size_t)p->capacity * 16 * sizeof(uint32_t)));
     PCU(p, cudaMalloc(&p->d_ns, (size_t)p->capacity * sizeof(uint64_t)));
-    PCU(p, cudaMalloc(&p->d_queue, (size_t)p->chunks * sizeof(uint32_t)));
-    PCU(p, cudaMalloc(&p->d_nq, 2 * sizeof(uint32_t)));
-    PCU(p, cudaMalloc(&p->d_chunk_search, (size_t)p->chunks * sizeof(uint32_t)));
-    PCU(p, cudaMalloc(&p->d_chunk_first, (size_t)p->chunks * sizeof(uint32_t)));
+    PCU(p, cudaMalloc(&p->d_queue, ((size_t)p->chunks + 1) * sizeof(uint4)));
     PCU(p, cudaMalloc(&p->d_searches, (size_t)p->max_searches * sizeof(lxk::PoolSearch)));
     PCU(p, cudaMalloc(&p->d_done, (size_t)p->chunks * sizeof(uint32_t)));
-    PCU(p, cudaMalloc(&p->d_hit_count, sizeof(uint32_t)));
-    PCU(p, cudaMalloc(&p->d_hits, (size_t)p->max_hits * sizeof(lxk::PoolHit)));
+    PCU(p, cudaMalloc(&p->d_hit_queue, ((size_t)p->max_hits + 1) * sizeof(lxk::PoolHit)));
     PCU(p, cudaMalloc(&p->d_scalars, (size_t)p->capacity * 32));
     PCU(p, cudaMalloc(&p->d_lane_map, (size_t)p->capacity * sizeof(uint32_t)));
-    PCU(p, cudaMallocHost(&p->h_hit_count, sizeof(uint32_t)));
-    PCU(p, cudaMallocHost(&p->h_hits, (size_t)p->max_hits * sizeof(lxk::PoolHit)));
-    *p->h_hit_count = 0;
-    PCU(p, cudaMemsetAsync(p->d_hit_count, 0, sizeof(uint32_t), p->stream));
-    PCU(p, cudaMemsetAsync(p->d_nq, 0, 2 * sizeof(uint32_t), p->stream));
+    PCU(p, cudaMallocHost(&p->h_hit_queue, p->first_bytes()));
+    memset(p->h_hit_queue, 0, p->first_bytes());
+    PCU(p, cudaMemsetAsync(p->d_hit_queue, 0, sizeof(uint32_t), p->stream));
     PCU(p, cudaMemsetAsync(p->d_done, 0, (size_t)p->chunks * sizeof(uint32_t), p->stream));
-    PCU(p, cudaMemsetAsync(p->d_chunk_search, 0, (size_t)p->chunks * sizeof(uint32_t), p->stream));
     p->chunk_owner.assign(p->chunks, -1);
-    p->h_chunk_search.assign(p->chunks, 0);
-    p->h_chunk_first.assign(p->chunks, 0);
+    p->h_queue.reserve((size_t)p->chunks + 1);
     p->free_chunks.resize(p->chunks);
     for (uint32_t c = 0; c < p->chunks; c++) p->free_chunks[c] = p->chunks - 1 - c;  // pop_back gives 0, 1, ...
     p->searches.resize(p->max_searches);
@@ -493,8 +484,6 @@ static int pool_submit_body(lxmfv_pool* p, const lxmfv_search_desc* d, const uin
     for (uint32_t i = 0; i < need; i++) {
         const uint32_t c = s.chunks[i];
         p->chunk_owner[c] = (int32_t)slot;
-        p->h_chunk_search[c] = slot;
-        p->h_chunk_first[c] = 32 * i;
         for (uint32_t j = 0; j < 32; j++) lane_map[32 * i + j] = 32 * c + j;
     }
     lxk::PoolSearch ps;
@@ -583,8 +572,6 @@ static int pool_submit_many_body(lxmfv_pool* p, const lxmfv_search_desc* descs, 
         for (uint32_t i = 0; i < d.lanes / 32; i++) {
             const uint32_t c = s.chunks[i];
             p->chunk_owner[c] = (int32_t)slot;
-            p->h_chunk_search[c] = slot;
-            p->h_chunk_first[c] = 32 * i;
             for (uint32_t j = 0; j < 32; j++) lane_map[at + 32 * i + j] = 32 * c + j;
         }
         at += d.lanes;
@@ -670,21 +657,25 @@ static int pool_step_body(lxmfv_pool* p, uint32_t groups) {
 
 int lxmfv_pool_poll(lxmfv_pool* p, lxmfv_pool_hit* hits, uint32_t cap, uint32_t* n_hits) {
     if (!p || !n_hits) return pfail(p, LXMFV_ERR_ARG, "null argument");
+    if (!p->h_hit_queue) return pfail(p, LXMFV_ERR_STATE, "the pool is not open");
     PCU(p, cudaSetDevice(p->device));
     PCU(p, cudaStreamSynchronize(p->stream));
-    // The last step's graph copied the hit queue to pinned memory.
-    const uint32_t count = *p->h_hit_count;
+    // The last step's graph copied the count and the first hits to pinned memory.
+    uint32_t count;
+    memcpy(&count, p->h_hit_queue, sizeof count);
     const uint32_t stored = std::min(count, p->max_hits);
     const uint32_t give = hits ? std::min(stored, cap) : 0;
-    for (uint32_t i = 0; i < give; i++) {
-        hits[i].search = p->h_hits[i].search;
-        hits[i].lane = p->h_hits[i].lane;
-        hits[i].n = p->h_hits[i].n;
+    const uint32_t here = std::min(give, kPoolFirstHits);
+    if (here) memcpy(hits, p->h_hit_queue + sizeof(lxk::PoolHit), sizeof(lxk::PoolHit) * here);
+    if (give > here) {
+        PCU(p, cudaMemcpyAsync(hits + here, p->hit_slots() + here, sizeof(lxk::PoolHit) * (give - here),
+                               cudaMemcpyDeviceToHost, p->stream));
+        PCU(p, cudaStreamSynchronize(p->stream));
     }
     *n_hits = count;
-    PCU(p, cudaMemsetAsync(p->d_hit_count, 0, sizeof(uint32_t), p->stream));
-    PCU(p, cudaStreamSynchronize(p->stream));
-    *p->h_hit_count = 0;
+    // Cleared in the stream's order, before any later step.
+    PCU(p, cudaMemsetAsync(p->d_hit_queue, 0, sizeof(uint32_t), p->stream));
+    memset(p->h_hit_queue, 0, sizeof(uint32_t));
     p->err.clear();
     return LXMFV_OK;
 }
@@ -733,17 +724,12 @@ void lxmfv_pool_close(lxmfv_pool* p) {
         cudaFree(p->d_state);
         cudaFree(p->d_ns);
         cudaFree(p->d_queue);
-        cudaFree(p->d_nq);
-        cudaFree(p->d_chunk_search);
-        cudaFree(p->d_chunk_first);
         cudaFree(p->d_searches);
         cudaFree(p->d_done);
-        cudaFree(p->d_hit_count);
-        cudaFree(p->d_hits);
+        cudaFree(p->d_hit_queue);
         cudaFree(p->d_scalars);
         cudaFree(p->d_lane_map);
-        cudaFreeHost(p->h_hit_count);
-        cudaFreeHost(p->h_hits);
+        cudaFreeHost(p->h_hit_queue);
         if (p->ev0) cudaEventDestroy(p->ev0);
         if (p->ev1) cudaEventDestroy(p->ev1);
         if (p->own_stream && p->stream) cudaStreamDestroy(p->stream);

@@ -100,6 +100,7 @@ class Pool:
             raise lx.LxmfvError(rc, msg)
         self.batch = batch
         self.max_hits = max_hits
+        self._hits = None
         self.specs: dict[int, SearchSpec] = {}
 
     def _check(self, rc: int) -> None:
@@ -163,7 +164,9 @@ class Pool:
 
     def poll(self, cap: int | None = None) -> tuple[list[tuple[int, int, int]], int]:
         cap = self.max_hits if cap is None else cap
-        hits = (lx.PoolHit * max(cap, 1))()
+        if self._hits is None or len(self._hits) < cap:
+            self._hits = (lx.PoolHit * max(cap, 1))()  # kept: clearing a megabyte for every step took longer than the poll
+        hits = self._hits
         n = C.c_uint32()
         self._check(lx.lib().lxmfv_pool_poll(self._h, hits, cap, C.byref(n)))
         got = min(n.value, cap)
