@@ -20,6 +20,25 @@ namespace lxk {
 
 constexpr int kCombThreads = 128;
 constexpr int kCombVecs = 32 * 8 * 24 / 4;  // uint4 of the table (24 KB)
+// A window's 48 uint4 at a stride of 49, so that threads at different windows
+// read different banks.
+constexpr int kCombStride = 49;
+constexpr int kCombShared = 32 * kCombStride;
+
+// Threads per scalar: one scalar's 64 additions and its inversion are a serial
+// chain of 0.18 ms, so few scalars are split over up to 16 threads, which take
+// every 16th window and add their sums up by shuffles, as long as every SM
+// sub-partition has a warp at most (more would only repeat the inversion).
+// 128 scalars on B200: 0.06 ms against 0.18; a serving turn that admits two
+// searches 4.63 -> 4.51 ms.
+inline uint32_t comb_threads(uint64_t scalars, uint32_t sms) {
+    uint32_t t = 1;
+    while (t < 16 && scalars * (2 * t) <= (uint64_t)sms * 128) t *= 2;
+    return t;
+}
+inline unsigned comb_blocks(uint64_t scalars, uint32_t threads) {
+    return (unsigned)((scalars * threads + kCombThreads - 1) / kCombThreads);
+}
 
 struct EdPoint {
     fe x, y, z, t;  // extended coordinates: x = X/Z, y = Y/Z, T = X Y / Z
@@ -28,7 +47,7 @@ struct EdPoint {
 // The table into shared memory; every thread of the block calls this.
 __device__ __forceinline__ void comb_stage(uint4* table) {
     const uint4* src = reinterpret_cast<const uint4*>(kCombTable);
-    for (int i = threadIdx.x; i < kCombVecs; i += blockDim.x) table[i] = src[i];
+    for (int i = threadIdx.x; i < kCombVecs; i += blockDim.x) table[i / 48 * kCombStride + i % 48] = src[i];
     __syncthreads();
 }
 
@@ -86,27 +105,52 @@ __device__ __forceinline__ void ed_double(EdPoint& p) {
     p.z = fe_mul(f, g);
 }
 
-// s Q for s < 2^255 (8 little-endian words).
-__device__ __forceinline__ EdPoint comb_mul(const uint32_t s[8], const uint4* table) {
+// p + q, both in extended coordinates (9 M).
+__device__ __forceinline__ EdPoint ed_add(const EdPoint& p, const EdPoint& q) {
+    constexpr uint32_t k2d[8] = LXK_COMB_2D;
+    fe d2;
+#pragma unroll
+    for (int i = 0; i < 8; i++) d2.v[i] = k2d[i];
+    const fe A = fe_mul(fe_sub(p.y, p.x), fe_sub(q.y, q.x));
+    const fe B = fe_mul(fe_add(p.y, p.x), fe_add(q.y, q.x));
+    const fe C = fe_mul(fe_mul(p.t, q.t), d2);
+    const fe zz = fe_mul(p.z, q.z), D = fe_add(zz, zz);
+    const fe E = fe_sub(B, A), F = fe_sub(D, C), G = fe_add(D, C), H = fe_add(B, A);
+    return EdPoint{fe_mul(E, F), fe_mul(G, H), fe_mul(F, G), fe_mul(E, H)};
+}
+
+__device__ __forceinline__ fe shfl_xor_fe(const fe& x, int m) {
+    fe r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = __shfl_xor_sync(0xffffffffu, x.v[i], m);
+    return r;
+}
+
+// s Q for s < 2^255 (8 little-endian words), by `threads` threads (a power of
+// two; thread t takes the windows t, t + threads, ...): every one gets it.
+__device__ __forceinline__ EdPoint comb_mul(const uint32_t s[8], const uint4* table, uint32_t t, uint32_t threads) {
     // s + 8 (1 + 16 + ... + 16^63): its nibbles less 8 are signed digits of s.
     uint32_t n[8], carry = 0;
 #pragma unroll
     for (int w = 0; w < 8; w++) {
-        const uint64_t t = (uint64_t)s[w] + 0x88888888u + carry;
-        n[w] = (uint32_t)t;
-        carry = (uint32_t)(t >> 32);
+        const uint64_t x = (uint64_t)s[w] + 0x88888888u + carry;
+        n[w] = (uint32_t)x;
+        carry = (uint32_t)(x >> 32);
     }
     EdPoint p{fe_zero(), fe_one(), fe_one(), fe_zero()};
 #pragma unroll 1
     for (int odd = 1; odd >= 0; odd--) {
 #pragma unroll 1
-        for (int i = 0; i < 32; i++)
-            comb_add(p, table + i * 48, (int)(n[i >> 2] >> (8 * (i & 3) + 4 * odd) & 15u) - 8);
+        for (uint32_t i = t; i < 32; i += threads)
+            comb_add(p, table + i * kCombStride, (int)(n[i >> 2] >> (8 * (i & 3) + 4 * odd) & 15u) - 8);
         if (odd) {
 #pragma unroll 1
             for (int i = 0; i < 4; i++) ed_double(p);
         }
     }
+#pragma unroll 1
+    for (uint32_t m = 1; m < threads; m *= 2)
+        p = ed_add(p, EdPoint{shfl_xor_fe(p.x, m), shfl_xor_fe(p.y, m), shfl_xor_fe(p.z, m), shfl_xor_fe(p.t, m)});
     return p;
 }
 
@@ -124,22 +168,38 @@ __device__ __forceinline__ void ed_to_affine_uv(const EdPoint& p, fe& u, fe& v) 
 
 // The centre C = (k/8 + m) Q of lane k's first group (walk indices 0 .. 2m-1).
 __device__ __forceinline__ void start_centre(const uint32_t* __restrict__ scalars, uint32_t i, uint32_t m,
-                                             const uint4* table, fe& u, fe& v) {
+                                             const uint4* table, uint32_t t, uint32_t threads, fe& u, fe& v) {
     uint32_t s[8];
     scalar_over_8(scalars, i, (int)m, s);
-    ed_to_affine_uv(comb_mul(s, table), u, v);
+    ed_to_affine_uv(comb_mul(s, table, t, threads), u, v);
+}
+
+// The scalar of a thread and its place among the scalar's threads; the last
+// block's spare threads repeat the last scalar (they take part in shuffles)
+// and store nothing.
+struct CombLane {
+    uint32_t i, t;
+    bool stores;
+};
+__device__ __forceinline__ CombLane comb_lane(uint32_t count, uint32_t threads) {
+    const uint64_t id = blockIdx.x * (uint64_t)kCombThreads + threadIdx.x;
+    const uint64_t i = id / threads;
+    const uint32_t t = (uint32_t)(id % threads);
+    return CombLane{i < count ? (uint32_t)i : count - 1, t, i < count && t == 0};
 }
 
 // Grouped walk from scalars.  75,776 lanes on B200: 0.47 ms, by the ladder 2.73; 128 lanes: 0.18 and 1.06.
 static __global__ void __launch_bounds__(kCombThreads) group_start_kernel(uint32_t* state, uint64_t* ns,
                                                                           const uint32_t* __restrict__ scalars,
-                                                                          uint32_t lanes, uint32_t m) {
-    __shared__ uint4 table[kCombVecs];
+                                                                          uint32_t lanes, uint32_t m,
+                                                                          uint32_t threads) {
+    __shared__ uint4 table[kCombShared];
     comb_stage(table);
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane >= lanes) return;
+    const CombLane c = comb_lane(lanes, threads);
+    const uint32_t lane = c.i;
     fe u, v;
-    start_centre(scalars, lane, m, table, u, v);
+    start_centre(scalars, lane, m, table, c.t, threads, u, v);
+    if (!c.stores) return;
     store_fe(state, 0, lane, lanes, u);
     store_fe(state, 1, lane, lanes, v);
     ns[lane] = 0;
@@ -147,10 +207,10 @@ static __global__ void __launch_bounds__(kCombThreads) group_start_kernel(uint32
 
 // P(-1) and P(0) of lane k, ((k - 8)B, kB), as u = X : Z.
 __device__ __forceinline__ void start_pair(const uint32_t* __restrict__ scalars, uint32_t lane, const uint4* table,
-                                           fe& x0, fe& z0, fe& x1, fe& z1) {
+                                           uint32_t t, uint32_t threads, fe& x0, fe& z0, fe& x1, fe& z1) {
     uint32_t s[8];
     scalar_over_8(scalars, lane, -1, s);
-    EdPoint p = comb_mul(s, table);
+    EdPoint p = comb_mul(s, table, t, threads);
     x0 = fe_add(p.z, p.y);
     z0 = fe_sub(p.z, p.y);
     comb_add(p, table, 1);  // + Q
@@ -162,13 +222,14 @@ __device__ __forceinline__ void start_pair(const uint32_t* __restrict__ scalars,
 // of first_public_keys, mod.rs:212-228, for the walk).
 static __global__ void __launch_bounds__(kCombThreads) xonly_start_kernel(uint32_t* state, uint64_t* ns,
                                                                           const uint32_t* __restrict__ scalars,
-                                                                          uint32_t lanes) {
-    __shared__ uint4 table[kCombVecs];
+                                                                          uint32_t lanes, uint32_t threads) {
+    __shared__ uint4 table[kCombShared];
     comb_stage(table);
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane >= lanes) return;
+    const CombLane c = comb_lane(lanes, threads);
+    const uint32_t lane = c.i;
     fe x0, z0, x1, z1;
-    start_pair(scalars, lane, table, x0, z0, x1, z1);
+    start_pair(scalars, lane, table, c.t, threads, x0, z0, x1, z1);
+    if (!c.stores) return;
     store_fe(state, 0, lane, lanes, x0);
     store_fe(state, 1, lane, lanes, z0);
     store_fe(state, 2, lane, lanes, x1);
@@ -182,13 +243,14 @@ static __global__ void __launch_bounds__(kCombThreads) xonly_start_kernel(uint32
 // the ladder 2.62.
 static __global__ void __launch_bounds__(kCombThreads) first_keys_kernel(uint4* __restrict__ upc,
                                                                          const uint32_t* __restrict__ scalars,
-                                                                         uint32_t lanes) {
-    __shared__ uint4 table[kCombVecs];
+                                                                         uint32_t lanes, uint32_t threads) {
+    __shared__ uint4 table[kCombShared];
     comb_stage(table);
-    const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lane >= lanes) return;
+    const CombLane c = comb_lane(lanes, threads);
+    const uint32_t lane = c.i;
     fe x0, z0, x1, z1;
-    start_pair(scalars, lane, table, x0, z0, x1, z1);
+    start_pair(scalars, lane, table, c.t, threads, x0, z0, x1, z1);
+    if (!c.stores) return;
     const fe inv = fe_invert(fe_mul(z0, z1));
     const fe u_prev = fe_canon(fe_mul(x0, fe_mul(inv, z1)));
     const fe u_cur = fe_canon(fe_mul(x1, fe_mul(inv, z0)));

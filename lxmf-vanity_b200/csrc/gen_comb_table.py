@@ -53,6 +53,7 @@ def main() -> None:
     print("#include <cstdint>")
     print()
     print(f"#define LXK_COMB_C {{{words(C)}}}")
+    print(f"#define LXK_COMB_2D {{{words(2 * D % P)}}}")
     print()
     print("static __device__ const uint32_t kCombTable[32 * 8 * 24] __attribute__((aligned(16))) = {")
     for _ in range(32):

@@ -602,12 +602,13 @@ int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_by
     uint32_t* d = w.take(n_bytes);
     cudaError_t e = cudaMemcpyAsync(d, scalars, n_bytes, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
+        const uint32_t t = lxk::comb_threads(h->lanes, (uint32_t)h->sms);
         if (h->walk == LXMFV_WALK_XADD) {
-            lxk::xonly_start_kernel<<<(h->lanes + 127) / 128, lxk::kCombThreads, 0, h->stream>>>(h->d_state, h->d_ns, d,
-                                                                                                 h->lanes);
+            lxk::xonly_start_kernel<<<lxk::comb_blocks(h->lanes, t), lxk::kCombThreads, 0, h->stream>>>(
+                h->d_state, h->d_ns, d, h->lanes, t);
         } else {
-            lxk::group_start_kernel<<<(h->lanes + 127) / 128, lxk::kCombThreads, 0, h->stream>>>(h->d_state, h->d_ns, d,
-                                                                                                 h->lanes, h->batch / 2);
+            lxk::group_start_kernel<<<lxk::comb_blocks(h->lanes, t), lxk::kCombThreads, 0, h->stream>>>(
+                h->d_state, h->d_ns, d, h->lanes, h->batch / 2, t);
         }
         e = cudaGetLastError();
     }
@@ -630,8 +631,9 @@ int lxmfv_first_public_keys(lxmfv_handle* h, const uint8_t* scalars, size_t coun
     uint32_t *ds = w.take(count * 32), *dout = w.take(count * 64);
     cudaError_t e = cudaMemcpyAsync(ds, scalars, count * 32, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
-        lxk::first_keys_kernel<<<(unsigned)((count + 127) / 128), lxk::kCombThreads, 0, h->stream>>>(
-            reinterpret_cast<uint4*>(dout), ds, (uint32_t)count);
+        const uint32_t t = lxk::comb_threads(count, (uint32_t)h->sms);
+        lxk::first_keys_kernel<<<lxk::comb_blocks(count, t), lxk::kCombThreads, 0, h->stream>>>(
+            reinterpret_cast<uint4*>(dout), ds, (uint32_t)count, t);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(u_prev_cur, dout, count * 64, cudaMemcpyDeviceToHost, h->stream);

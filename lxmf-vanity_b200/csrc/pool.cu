@@ -143,14 +143,14 @@ static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(co
 static __global__ void __launch_bounds__(kCombThreads) pool_start_kernel(uint32_t* state, uint64_t* ns, uint32_t capacity,
                                                                  const uint32_t* __restrict__ scalars,
                                                                  const uint32_t* __restrict__ lane_map, uint32_t count,
-                                                                 uint32_t m) {
-    __shared__ uint4 table[kCombVecs];
+                                                                 uint32_t m, uint32_t threads) {
+    __shared__ uint4 table[kCombShared];
     comb_stage(table);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    const CombLane c = comb_lane(count, threads);
     fe u, v;
-    start_centre(scalars, i, m, table, u, v);
-    const uint32_t lane = lane_map[i];
+    start_centre(scalars, c.i, m, table, c.t, threads, u, v);
+    if (!c.stores) return;
+    const uint32_t lane = lane_map[c.i];
     store_fe(state, 0, lane, capacity, u);
     store_fe(state, 1, lane, capacity, v);
     ns[lane] = 0;
@@ -498,8 +498,9 @@ static int pool_submit_body(lxmfv_pool* p, const lxmfv_search_desc* d, const uin
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(p->d_lane_map, lane_map.data(), sizeof(uint32_t) * d->lanes, cudaMemcpyHostToDevice, p->stream);
     if (e == cudaSuccess) {
-        lxk::pool_start_kernel<<<(d->lanes + 127) / 128, lxk::kCombThreads, 0, p->stream>>>(
-            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, d->lanes, p->m);
+        const uint32_t t = lxk::comb_threads(d->lanes, (uint32_t)p->sms);
+        lxk::pool_start_kernel<<<lxk::comb_blocks(d->lanes, t), lxk::kCombThreads, 0, p->stream>>>(
+            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, d->lanes, p->m, t);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
@@ -597,8 +598,9 @@ static int pool_submit_many_body(lxmfv_pool* p, const lxmfv_search_desc* descs, 
         e = cudaMemcpyAsync(p->d_lane_map, lane_map.data(), sizeof(uint32_t) * lanes_total, cudaMemcpyHostToDevice,
                             p->stream);
     if (e == cudaSuccess) {
-        lxk::pool_start_kernel<<<(unsigned)((lanes_total + 127) / 128), lxk::kCombThreads, 0, p->stream>>>(
-            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, (uint32_t)lanes_total, p->m);
+        const uint32_t t = lxk::comb_threads(lanes_total, (uint32_t)p->sms);
+        lxk::pool_start_kernel<<<lxk::comb_blocks(lanes_total, t), lxk::kCombThreads, 0, p->stream>>>(
+            p->d_state, p->d_ns, p->capacity, p->d_scalars, p->d_lane_map, (uint32_t)lanes_total, p->m, t);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) {

@@ -514,3 +514,19 @@ def test_xonly_units_agree_with_the_grouped_walk(lx, lanes, batch):
                 hits.update(h)
             got.append(hits)
     assert got[0] == got[1] and got[0]
+
+
+@pytest.mark.parametrize("count", [1185, 2369, 4737, 9473])
+def test_start_points_over_several_threads(lx, count):
+    """A scalar over 8, 4, 2 and 1 threads (the smallest counts of each on 148
+    SMs; fewer scalars take 16), against OpenSSL's X25519 for some of them and
+    against 16 threads each for 900 of them."""
+    scal, _ = lx.seeded_scalars(count, 0, count)
+    with lx.Backend(device=0, lanes=32) as b:
+        pair = b.first_public_keys(scal)
+        back = b.first_public_keys(scal[::-1][:900])  # 16 threads each
+    assert (back == pair[::-1][:900]).all()
+    u = pair.view(np.uint8).reshape(count, 2, 32)
+    for t in list(range(0, count, count // 12)) + [count - 1]:
+        assert bytes(u[t, 1]) == lx.x25519_base(bytes(scal[t]))
+        assert bytes(u[t, 0]) == lx.x25519_base(lx.previous_scalar(bytes(scal[t])))
