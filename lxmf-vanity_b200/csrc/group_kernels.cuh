@@ -275,7 +275,7 @@ inline uint32_t group_parts(uint64_t chunks, uint32_t m, uint32_t sms) {
         const uint64_t units = chunks * s, rest = units % slots;
         const uint64_t rounds = units / slots * kRound[4] + kRound[(rest + 4 * sms - 1) / (4 * sms)];
         const uint64_t cost = (10 * ((m + s - 1) / s) + 18) * rounds;
-        if (cost < best_cost) {
+        if (cost <= best_cost) {  // of equals the larger: some of its parts have a pair less
             best_cost = cost;
             best = s;
         }
