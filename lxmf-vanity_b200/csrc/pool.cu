@@ -87,9 +87,9 @@ struct PoolEmit {
     __device__ __forceinline__ void operator()(const fe& u, uint64_t key) const {
         uint32_t d[4];
         lxsha::dest_hash_one(u.v, ac.ed, ac, one, d);
-        const bool match = ((d[0] & ac.mask[0]) == ac.want[0]) & ((d[1] & ac.mask[1]) == ac.want[1]) &
-                           ((d[2] & ac.mask[2]) == ac.want[2]) & ((d[3] & ac.mask[3]) == ac.want[3]);
-        if (match) {
+        if ((d[0] & ac.mask[0]) == ac.want[0] &&
+            ((d[1] & ac.mask[1]) == ac.want[1]) & ((d[2] & ac.mask[2]) == ac.want[2]) &
+                ((d[3] & ac.mask[3]) == ac.want[3])) {
             const uint32_t slot = atomicAdd(hit_count, 1u);
             if (slot < max_hits) {
                 hits[slot].search = search;

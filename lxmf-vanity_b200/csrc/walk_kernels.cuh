@@ -79,9 +79,9 @@ template <bool DUMP>
 __device__ __forceinline__ void emit_key(const EmitArgs& a, uint32_t lane, uint64_t key, uint64_t key0, const fe& u) {
     uint32_t d[4];
     lxsha::dest_hash(u.v, a.ac.ed, a.ac, d);
-    const bool match = ((d[0] & a.ac.mask[0]) == a.ac.want[0]) & ((d[1] & a.ac.mask[1]) == a.ac.want[1]) &
-                       ((d[2] & a.ac.mask[2]) == a.ac.want[2]) & ((d[3] & a.ac.mask[3]) == a.ac.want[3]);
-    if (match) {
+    if ((d[0] & a.ac.mask[0]) == a.ac.want[0] &&
+        ((d[1] & a.ac.mask[1]) == a.ac.want[1]) & ((d[2] & a.ac.mask[2]) == a.ac.want[2]) &
+            ((d[3] & a.ac.mask[3]) == a.ac.want[3])) {
         const uint32_t slot = atomicAdd(a.hit_count, 1u);
         if (slot < a.max_hits) {
             a.hits[slot].thread = lane;
