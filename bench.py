@@ -49,38 +49,36 @@ METRIC = "keys/s, plain GPU search (one 8-hex prefix, seeded walkers, 2^36 keys)
 
 
 def field_ops_per_key(walk: str, b: int) -> tuple[float, float]:
-    """(multiplies, squarings) per key, counted from the kernels' code.
-    x-only walk, B keys per inversion: 8B + 11 M and 2B + 254 S per batch.
-    Grouped walk, G = 2m keys per group: (5m + 13) M and (2m + 255) S per group."""
+    """(multiplies, squarings) per key, counted from the kernels' code; the
+    inversion (by divsteps) is neither.  x-only walk: 8B M and 2B S per batch.
+    Grouped walk, G = 2m keys per group: (5m + 2) M and (2m + 1) S per group."""
     if walk == "xadd":
-        return 8 + 11 / b, 2 + 254 / b
+        return 8.0, 2.0
     m = b // 2
-    return (5 * m + 13) / b, (2 * m + 255) / b
+    return (5 * m + 2) / b, (2 * m + 1) / b
 
 
-# Per key, from ncu captures of each kernel on a small case (profiles/walk_group_g1024_plain_search.md,
-# profiles/walk_group_g64_plain_search.md, profiles/walk_xadd_b64_plain_search.md; the G = 512, 256 and x-only
-# B = 128 rows from the earlier captures in profiles/):
-#   alu: ALU-pipe lane operations (the binding pipe): sm__inst_executed_pipe_alu.sum x 32 / keys (earlier rows:
-#        ALU pipe active % x 64 lanes x SMs x clock / keys per second);
+# Per key, from ncu captures of each kernel on a small case (profiles/pipe_counts_plain_search.md):
+#   alu: ALU-pipe lane operations (the binding pipe): sm__inst_executed_pipe_alu.sum x 32 / keys;
 #   imad: IMAD-class instructions per key: sm__inst_executed_pipe_fmaheavy.sum x 32 / keys, the pipe that
 #        executes IMAD, IMAD.HI, IMAD.WIDE and IMAD.X (these kernels run no floating point);
 #   inst: all instructions (smsp__inst_executed.sum x 32 / keys); dram_bytes: DRAM read + write.
 NCU_PER_KEY = {
-    ("group", 1024): {"alu": 3213, "imad": 2219, "inst": 5764, "dram_bytes": 32.0},
-    ("group", 512): {"alu": 3243, "inst": 5823, "dram_bytes": 31.6},
-    ("group", 256): {"alu": 3288, "inst": 5935, "dram_bytes": 31.1},
-    ("group", 64): {"alu": 3546, "imad": 2678, "inst": 6605, "dram_bytes": 24.8},
-    ("xadd", 128): {"alu": 4166, "inst": 8120, "dram_bytes": 131.9},
-    ("xadd", 64): {"alu": 4319, "imad": 3740, "inst": 8562, "dram_bytes": 132.1},
+    ("group", 1024): {"alu": 2844, "imad": 1902, "inst": 4939, "dram_bytes": 31.4},
+    ("group", 512): {"alu": 2850, "imad": 1912, "inst": 4955, "dram_bytes": 30.5},
+    ("group", 256): {"alu": 2862, "imad": 1932, "inst": 4988, "dram_bytes": 29.3},
+    ("group", 64): {"alu": 2938, "imad": 2055, "inst": 5191, "dram_bytes": 10.4},
+    ("xadd", 128): {"alu": 3146, "imad": 2435, "inst": 5794, "dram_bytes": 121.4},
+    ("xadd", 64): {"alu": 3203, "imad": 2503, "inst": 5921, "dram_bytes": 114.5},
 }
 
 
 def wide_products_per_key(walk: str, b: int) -> float:
-    """32x32->64 products per key with 8 x 32-bit limbs: a field multiply is
-    64 + 8 (the fold by 38), a square 36 + 8."""
+    """32x32->64 products per key: with 8 x 32-bit limbs a field multiply is
+    64 + 8 (the fold by 38), a square 36 + 8; an inversion per b keys is 20
+    batches of 76 on 9 x 30-bit limbs (fe_divsteps.h)."""
     mul, sqr = field_ops_per_key(walk, b)
-    return mul * 72 + sqr * 44
+    return mul * 72 + sqr * 44 + 20 * 76 / b
 
 
 def parse() -> argparse.Namespace:
@@ -385,9 +383,9 @@ def main() -> None:
         # The same workload at B = 64 keys per inversion, the reference kernel's
         # batch: the grouped walk, then the x-only walk (the reference's
         # algorithm: xADD by Q and Montgomery batch inversion over 64 keys).
-        # Each in its fastest launch shape (the autotuner's): the x-only walk runs
-        # without the phase barrier, 3% faster than with it.
-        for key, walk, shape in (("at_batch_64", "group", None), ("xadd_b64", "xadd", (512, False))):
+        # Each in the library's default launch shape for it, the fastest over
+        # launches this long (the phase barrier at both).
+        for key, walk, shape in (("at_batch_64", "group", None), ("xadd_b64", "xadd", None)):
             r = measure(torch, dist, lx, a, dev, rank, world, prefix, walk, 64, a.total_keys, a.steps, a.warmup,
                         e2e=False, shape=shape)
             line[key] = {"value": r["value"], "unit": "keys/s", "ms_per_step": r["ms_per_step"],
@@ -547,7 +545,8 @@ def measure(torch, dist, lx, a, dev, rank, world, prefix, walk, batch, total_key
         roofline = dict(imad_line, bound="imad", traffic=None, alu_peak=alu_peak / 1e12)
     config = {"workload": "plain GPU search (8-hex prefix, lxmf.delivery, seeded walkers, 2^36 keys per run)",
               "walk": walk, "prefix": prefix, "lanes_per_gpu": lanes, "batch": batch, "iters_per_step": iters,
-              "block": block or 512, "phase_barrier": bool(flags) if block else True,
+              "block": block or 512,
+              "phase_barrier": bool(flags) if block else batch < (256 if walk == "group" else 128),
               "keys_per_step_per_gpu": keys_per_step, "parallelism": f"replicas x{world}",
               "l2": "working set (lane state + per-lane batch buffers) exceeds L2; no flush needed"}
     rank_record = {"rank": rank, "device": dev, "seed": replicas.rank_seed(SEED, rank), "ms": ms_rank,

@@ -76,7 +76,7 @@ typedef struct {
     uint32_t lanes;       /* walker lanes (GPU threads); 0: one full wave of the device */
     uint32_t batch;       /* keys per inversion: XADD 16, 32, 64, 128; GROUP 32 .. 1024; 0: the fastest (GROUP 1024, XADD 128) */
     uint32_t block;       /* threads per block: 128, 256 or 512; 0: 512, with LXMFV_FLAG_PHASE_SYNC where batches
-                           * are short (GROUP below 256, XADD below 64: the faster, measured).  It holds for
+                           * are short (GROUP below 256, XADD below 128: the faster, measured).  It holds for
                            * lanes in whole waves (512 per SM); other counts are walked in a shape of the library's own,
                            * the grouped walk's in parts, several warps per 32 lanes (not with REGCAP_80 or WARP_SPEC) */
     uint32_t walk;        /* LXMFV_WALK_GROUP (0, default) or LXMFV_WALK_XADD */

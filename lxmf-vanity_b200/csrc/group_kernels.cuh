@@ -337,9 +337,9 @@ static __global__ void __launch_bounds__(BLOCK, MINB) group_walk_kernel(const __
 // The plain walk in parts: one block per SM, whose warps take units of (32
 // lanes, part) a grid apart, so that the units of a short last round spread
 // over all SMs and their sub-partitions.  Lanes past the last one walk a copy
-// of it.  At G = 1024 on B200, one group: 32 lanes 15.2 -> 0.08 ms, 2,048
-// lanes 15.2 -> 0.54 ms, 100,003 lanes 30.3 -> 20.5 ms (5.00 G keys/s; a whole
-// wave 5.11).
+// of it.  At G = 1024 on B200, one group: 32 lanes 0.04 ms, 2,048 lanes
+// 0.46, 100,003 lanes 19.9 (5.15 G keys/s; a whole wave 5.26); one warp per
+// chunk in blocks of 512: 15, 15 and 30 ms.
 template <int M, bool DUMP, class Args = GroupArgsFor<M>>
 static __global__ void __launch_bounds__(32 * kPartsWarps, 1) group_parts_kernel(const __grid_constant__ Args a) {
     const uint32_t lid = threadIdx.x & 31;

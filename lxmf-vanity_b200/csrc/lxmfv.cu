@@ -468,12 +468,14 @@ int lxmfv_open(const lxmfv_options* opts, lxmfv_handle** out) {
     // 0: the fastest keys per inversion of each walk (the autotuner's choice).
     h->batch = o.batch ? o.batch : (o.walk == LXMFV_WALK_XADD ? 128 : 1024);
     // Default launch shape (block 0): 512 threads, with the phase barrier where
-    // batches are short; otherwise the flags decide.  Measured on B200 over two
-    // waves of lanes, G keys/s without and with it: grouped walk G = 64 4.92,
-    // 4.96; G = 128 5.10, 5.10; G = 256 5.19, 5.17; G = 1024 5.25, 5.22; x-only
-    // walk B = 32 3.62, 3.76; B = 64 3.92, 3.91; B = 128 4.05, 3.99.
+    // batches are short; otherwise the flags decide.  Measured on B200 over
+    // launches of 2^28 and 2^31 keys (two waves of lanes), G keys/s without and
+    // with it: grouped walk G = 64 4.94 and 4.92, 4.97; G = 128 5.10, 5.10; G = 256
+    // 5.19 and 5.21, 5.17; G = 1024 5.25 and 5.27, 5.23; x-only walk B = 32 3.63 and
+    // 3.57, 3.77; B = 64 3.93 and 3.80 (its warps drift apart in a long launch),
+    // 3.91; B = 128 4.05 and 4.00, 3.99.
     h->block = o.block ? o.block : 512;
-    h->sync = o.block ? (o.flags & LXMFV_FLAG_PHASE_SYNC) != 0 : h->batch < (o.walk == LXMFV_WALK_XADD ? 64u : 256u);
+    h->sync = o.block ? (o.flags & LXMFV_FLAG_PHASE_SYNC) != 0 : h->batch < (o.walk == LXMFV_WALK_XADD ? 128u : 256u);
     h->low_regs = (o.flags & LXMFV_FLAG_REGCAP_80) != 0;
     h->ws = (o.flags & LXMFV_FLAG_WARP_SPEC) != 0;
     if (h->ws && (h->walk != LXMFV_WALK_GROUP || !ws_kernel_for(h->batch, false) || h->low_regs ||

@@ -103,8 +103,9 @@ struct PoolEmit {
 // No barrier: the warps of a block start together and do equal work, so they
 // stay in one phase of the walk by themselves.  In items of 16 chunks per block
 // with a phase barrier, 636 chunks kept 40 of 148 SMs busy for 16.3 ms per group
-// of 1024; in parts, as units of a warp, they take 4.6 ms.  The full pool (9,472
-// chunks, one part) walks 5.08 G keys/s, 5.12 in items of 16.
+// of 1024; in parts, as units of a warp, they take 4.3 ms.  The full pool (9,472
+// chunks, one part) walks 5.23 G keys/s (as units of a warp 0.6% less than in
+// items of 16, measured with the field code before the canonical sums).
 template <int M>
 static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(const __grid_constant__ PoolArgs<M> a) {
     __shared__ lxsha::AddrConsts s_ac[kPoolWarps];
