@@ -269,6 +269,7 @@ constexpr int kPartsWarps = 16;  // warps per block (512 threads, one block per 
 inline uint32_t group_parts(uint64_t chunks, uint32_t m, uint32_t sms) {
     static const uint32_t kRound[5] = {0, 21, 34, 49, 64};
     const uint64_t slots = (uint64_t)sms * kPartsWarps;
+    if (slots == 0) return 1;  // a handle that failed to open
     uint32_t best = 1;
     uint64_t best_cost = ~0ull;
     for (uint32_t s = 1; s <= m; s++) {

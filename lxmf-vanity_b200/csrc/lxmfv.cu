@@ -697,6 +697,7 @@ int lxmfv_collect(lxmfv_handle* h, lxmfv_hit* hits, uint32_t hits_cap, uint32_t*
                   uint32_t* dump_addr) {
     if (!h || !n_hits) return fail(h, LXMFV_ERR_ARG, "null argument");
     if (int rc = set_device(h)) return rc;
+    if (!h->d_hit_queue) return fail(h, LXMFV_ERR_CUDA, "handle is not open");
     // The count and the first hits come in one copy; a search rarely has more.
     constexpr uint32_t kFirst = 255;
     lxk::Hit first[kFirst + 1];
@@ -779,6 +780,7 @@ int lxmfv_fe_op(lxmfv_handle* h, int op, const uint32_t* a, const uint32_t* b, u
     if (op == 3 && (group < 1 || group > 256)) return fail(h, LXMFV_ERR_ARG, "group %u not in 1..256", group);
     if (count == 0) return LXMFV_OK;
     if (count > kMaxArray) return fail(h, LXMFV_ERR_CUDA, "fe_op: out of memory");
+    if (!h->sms) return fail(h, LXMFV_ERR_CUDA, "fe_op: handle is not open");
     if (int rc = set_device(h)) return rc;
     const size_t bytes = count * 8 * sizeof(uint32_t);
     Work w;

@@ -294,7 +294,7 @@ void launch_pool_any(lxmfv_pool* p, uint32_t groups) {
 int rebuild_queue(lxmfv_pool* p) {
     auto& q = p->h_queue;
     q.assign(1, make_uint4(0, 0, 0, 0));
-    for (uint32_t slot = 0; slot < p->max_searches; slot++) {
+    for (uint32_t slot = 0; slot < p->searches.size(); slot++) {
         const auto& s = p->searches[slot];
         if (s.active)
             for (uint32_t i = 0; i < s.chunks.size(); i++) q.push_back(make_uint4(s.chunks[i], slot, 32 * i, 0));
@@ -644,6 +644,7 @@ static int pool_retire_body(lxmfv_pool* p, uint32_t search_id) {
 static int pool_step_body(lxmfv_pool* p, uint32_t groups) {
     if (!p) return LXMFV_ERR_ARG;
     if (groups == 0 || groups > (1u << 16)) return pfail(p, LXMFV_ERR_ARG, "groups %u: 1 .. 65536", groups);
+    if (!p->h_hit_queue) return pfail(p, LXMFV_ERR_CUDA, "the pool is not open");
     PCU(p, cudaSetDevice(p->device));
     if (p->queue_dirty)
         if (int rc = rebuild_queue(p)) return rc;
