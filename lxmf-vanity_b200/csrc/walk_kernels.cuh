@@ -203,6 +203,7 @@ static __global__ void init_kernel(uint32_t* state, uint64_t* ns, const uint32_t
 // The Montgomery ladder (RFC 7748's step, a24 = 121665, swaps by masks: no
 // branch on a secret bit) over bits [nbits-1, 0] of the 256-bit scalar s
 // (8 LE words), base point u = q: ends with (X2:Z2) = s Q, (X3:Z3) = (s+1) Q.
+// The group table's multiples come from it; start points do not (comb_kernels.cuh).
 __device__ __forceinline__ void ladder(const uint32_t s[8], int nbits, const fe& q, fe& x2, fe& z2, fe& x3, fe& z3) {
     x2 = fe_one();
     z2 = fe_zero();

@@ -409,7 +409,7 @@ class Backend:
         self._check(lib().lxmfv_init(self._h, a.ctypes.data_as(_u32p), a.size))
 
     def init_from_scalars(self, scalars: np.ndarray | bytes) -> None:
-        """Start points by the GPU ladder from 32-byte clamped scalars."""
+        """Start points on the GPU from 32-byte clamped scalars."""
         a = np.frombuffer(scalars, np.uint8) if isinstance(scalars, (bytes, bytearray)) else \
             np.ascontiguousarray(scalars, np.uint8).reshape(-1)
         self._check(lib().lxmfv_init_from_scalars(self._h, a.ctypes.data_as(_u8p), a.size))
