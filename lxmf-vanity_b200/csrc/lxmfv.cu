@@ -51,6 +51,7 @@ struct lxmfv_handle {
     uint32_t launch_max_hits = 0;            // largest max_hits since the last collect
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool timed = false;
+    bool opened = false;       // lxmfv_open ended well: every buffer and table is there
     bool initialised = false;
     fe tu[LXMFV_MAX_HALF_GROUP + 1], tv[LXMFV_MAX_HALF_GROUP + 1];  // grouped walk: J, 1Q .. MQ
     std::string err;
@@ -74,6 +75,13 @@ int fail(lxmfv_handle* h, int code, const char* fmt, ...) {
         if (e_ != cudaSuccess)                                                               \
             return fail((h), LXMFV_ERR_CUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), \
                         __FILE__, __LINE__);                                                 \
+    } while (0)
+
+// Every call that works on the device asks first: after an open that failed
+// part-way some buffers or the group table are missing.
+#define NEED_OPEN(h, code)                                                \
+    do {                                                                  \
+        if (!(h)->opened) return fail((h), (code), "handle is not open"); \
     } while (0)
 
 constexpr int minb(int block) { return block == 512 ? 1 : block == 256 ? 2 : 4; }
@@ -549,6 +557,7 @@ int lxmfv_open(const lxmfv_options* opts, lxmfv_handle** out) {
     if (h->walk == LXMFV_WALK_GROUP)
         if (int rc = build_group_table(h)) return rc;
     CU(h, cudaStreamSynchronize(h->stream));
+    h->opened = true;
     h->err.clear();
     return LXMFV_OK;
 }
@@ -568,7 +577,7 @@ uint32_t lxmfv_walk(const lxmfv_handle* h) { return h ? h->walk : 0; }
 
 int lxmfv_init(lxmfv_handle* h, const uint32_t* u_prev_cur, size_t n_words) {
     if (!h || !u_prev_cur) return fail(h, LXMFV_ERR_ARG, "null argument");
-    if (!h->d_state) return fail(h, LXMFV_ERR_STATE, "handle is not open");
+    NEED_OPEN(h, LXMFV_ERR_STATE);
     if (n_words != (size_t)h->lanes * 16)
         return fail(h, LXMFV_ERR_ARG, "u_prev_cur has %zu words; %u lanes need %zu", n_words, h->lanes,
                     (size_t)h->lanes * 16);
@@ -596,7 +605,7 @@ int lxmfv_init(lxmfv_handle* h, const uint32_t* u_prev_cur, size_t n_words) {
 
 int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_bytes) {
     if (!h || !scalars) return fail(h, LXMFV_ERR_ARG, "null argument");
-    if (!h->d_state) return fail(h, LXMFV_ERR_STATE, "handle is not open");
+    NEED_OPEN(h, LXMFV_ERR_STATE);
     if (n_bytes != (size_t)h->lanes * 32)
         return fail(h, LXMFV_ERR_ARG, "scalars have %zu bytes; %u lanes need %zu", n_bytes, h->lanes,
                     (size_t)h->lanes * 32);
@@ -626,7 +635,7 @@ int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_by
 
 int lxmfv_first_public_keys(lxmfv_handle* h, const uint8_t* scalars, size_t count, uint32_t* u_prev_cur) {
     if (!h || !scalars || !u_prev_cur) return fail(h, LXMFV_ERR_ARG, "null argument");
-    if (!h->sms) return fail(h, LXMFV_ERR_STATE, "handle is not open");
+    NEED_OPEN(h, LXMFV_ERR_STATE);
     if (count == 0) return LXMFV_OK;
     if (count > (1u << 30)) return fail(h, LXMFV_ERR_ARG, "count %zu too large", count);
     if (int rc = check_scalars(h, scalars, count)) return rc;
@@ -696,8 +705,8 @@ int lxmfv_launch_async(lxmfv_handle* h, const lxmfv_launch_args* args) {
 int lxmfv_collect(lxmfv_handle* h, lxmfv_hit* hits, uint32_t hits_cap, uint32_t* n_hits, uint32_t* dump,
                   uint32_t* dump_addr) {
     if (!h || !n_hits) return fail(h, LXMFV_ERR_ARG, "null argument");
+    NEED_OPEN(h, LXMFV_ERR_CUDA);
     if (int rc = set_device(h)) return rc;
-    if (!h->d_hit_queue) return fail(h, LXMFV_ERR_CUDA, "handle is not open");
     // The count and the first hits come in one copy; a search rarely has more.
     constexpr uint32_t kFirst = 255;
     lxk::Hit first[kFirst + 1];
@@ -780,7 +789,7 @@ int lxmfv_fe_op(lxmfv_handle* h, int op, const uint32_t* a, const uint32_t* b, u
     if (op == 3 && (group < 1 || group > 256)) return fail(h, LXMFV_ERR_ARG, "group %u not in 1..256", group);
     if (count == 0) return LXMFV_OK;
     if (count > kMaxArray) return fail(h, LXMFV_ERR_CUDA, "fe_op: out of memory");
-    if (!h->sms) return fail(h, LXMFV_ERR_CUDA, "fe_op: handle is not open");
+    NEED_OPEN(h, LXMFV_ERR_CUDA);
     if (int rc = set_device(h)) return rc;
     const size_t bytes = count * 8 * sizeof(uint32_t);
     Work w;
@@ -811,6 +820,7 @@ int lxmfv_address_chain(lxmfv_handle* h, const uint8_t* pks, const uint8_t name_
     if (!h || !pks || !name_hash || !out) return fail(h, LXMFV_ERR_ARG, "null argument");
     if (count == 0) return LXMFV_OK;
     if (count > kMaxArray) return fail(h, LXMFV_ERR_CUDA, "address_chain: out of memory");
+    NEED_OPEN(h, LXMFV_ERR_CUDA);
     if (int rc = set_device(h)) return rc;
     uint32_t nh[3] = {(uint32_t)name_hash[0] << 24 | (uint32_t)name_hash[1] << 16 | (uint32_t)name_hash[2] << 8 | name_hash[3],
                       (uint32_t)name_hash[4] << 24 | (uint32_t)name_hash[5] << 16 | (uint32_t)name_hash[6] << 8 | name_hash[7],
@@ -833,6 +843,7 @@ int lxmfv_address_chain(lxmfv_handle* h, const uint8_t* pks, const uint8_t name_
 
 int lxmfv_peak_probe(lxmfv_handle* h, int kind, float ms, double* ops_per_s) {
     if (!h || !ops_per_s || kind < 0 || kind > 7) return fail(h, LXMFV_ERR_ARG, "bad argument");
+    NEED_OPEN(h, LXMFV_ERR_CUDA);
     if (int rc = set_device(h)) return rc;
     uint32_t* sink = nullptr;
     CU(h, cudaMalloc(&sink, sizeof(uint32_t)));

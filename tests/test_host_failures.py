@@ -1,0 +1,107 @@
+"""The library's host code over a CUDA runtime without a device
+(fake_cudart.c, linked with the library's own objects): what an allocation
+that fails leaves open, and what stays behind in device memory.  No GPU."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA_INCLUDE = "/usr/local/cuda/include"
+
+
+@pytest.fixture(scope="module")
+def fake(lx, tmp_path_factory):
+    import build as lxbuild
+
+    lxbuild.build()
+    so = str(tmp_path_factory.mktemp("fake") / "liblxmfv_fake.so")
+    objs = [os.path.join(lxbuild.OBJ, s + ".o") for s in lxbuild.CU_SOURCES + lxbuild.CXX_SOURCES]
+    obj = so + ".o"
+    subprocess.run(["gcc", "-O1", "-fPIC", "-I", CUDA_INCLUDE, "-c", os.path.join(HERE, "fake_cudart.c"), "-o", obj], check=True)
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", so, obj] + objs + ["-lcrypto"], check=True)
+    L = C.CDLL(so)
+    for name in ("fake_used",):
+        getattr(L, name).restype = C.c_size_t
+    L.fake_set_capacity.argtypes = [C.c_size_t]
+    L.fake_holds.argtypes = [C.c_char_p, C.c_size_t]
+    L.lxmfv_pool_keys_per_lane.restype = C.c_uint64
+    for name in ("lxmfv_close", "lxmfv_pool_close"):
+        getattr(L, name).restype = None
+    L.fake_reset()
+    yield L
+    L.fake_reset()
+
+
+def _u8(a):
+    return a.ctypes.data_as(C.POINTER(C.c_uint8))
+
+
+def _u32(a):
+    return a.ctypes.data_as(C.POINTER(C.c_uint32))
+
+
+def _handle_calls(lx, L, h, lanes):
+    """Every entry point that works on a handle, with arguments that an open
+    one accepts."""
+    scal, _ = lx.seeded_scalars(3, 0, lanes)
+    words = np.ones((lanes, 16), np.uint32)
+    a, out = np.ones((64, 8), np.uint32), np.zeros((64, 8), np.uint32)
+    pks, addr = np.zeros((64, 64), np.uint8), np.zeros((64, 16), np.uint8)
+    args = lx.make_launch_args(1, bytes(32), lx.prefix_parse("b0"))
+    n, d = C.c_uint32(), C.c_double()
+    nh = (C.c_uint8 * 10)()
+    yield "init", lambda: L.lxmfv_init(h, _u32(words), C.c_size_t(words.size))
+    yield "init_from_scalars", lambda: L.lxmfv_init_from_scalars(h, _u8(scal), C.c_size_t(32 * lanes))
+    yield "first_public_keys", lambda: L.lxmfv_first_public_keys(h, _u8(scal), C.c_size_t(lanes), _u32(words))
+    yield "launch_async", lambda: L.lxmfv_launch_async(h, C.byref(args))
+    yield "collect", lambda: L.lxmfv_collect(h, None, 0, C.byref(n), None, None)
+    yield "launch", lambda: L.lxmfv_launch(h, C.byref(args), None, 0, C.byref(n), None, None)
+    for op in range(4):
+        yield f"fe_op {op}", lambda op=op: L.lxmfv_fe_op(h, op, _u32(a), _u32(a), _u32(out), C.c_uint64(64), 8)
+    yield "address_chain", lambda: L.lxmfv_address_chain(h, _u8(pks), nh, _u8(addr), C.c_uint64(64))
+    yield "peak_probe", lambda: L.lxmfv_peak_probe(h, 0, C.c_float(1.0), C.byref(d))
+
+
+@pytest.mark.parametrize("walk,batch", [(0, 64), (0, 1024), (1, 64)])
+def test_a_handle_whose_open_failed_at_any_allocation(lx, fake, walk, batch):
+    """Every allocation of lxmfv_open fails in turn: open says so, every call
+    on the handle is refused before any launch, and close leaves nothing."""
+    lanes = 96
+    for at in range(64):
+        fake.fake_reset()
+        fake.fake_fail_after(at)
+        h = C.c_void_p()
+        rc = fake.lxmfv_open(C.byref(lx.Options(0, lanes, batch, 0, walk, 0, None)), C.byref(h))
+        if fake.fake_pending():  # open made fewer allocations than that
+            assert rc == lx.OK
+            fake.fake_reset()
+            for name, call in _handle_calls(lx, fake, h, lanes):
+                assert call() == lx.OK, name
+            fake.lxmfv_close(h)
+            assert fake.fake_used() == 0
+            break
+        assert rc == lx.ERR_CUDA, at
+        before = fake.fake_launches()
+        for name, call in _handle_calls(lx, fake, h, lanes):
+            assert call() != lx.OK, (at, name)
+            assert fake.fake_launches() == before, (at, name)
+        fake.lxmfv_close(h)
+        assert fake.fake_used() == 0, at
+    else:
+        pytest.fail("open never succeeded")
+    assert at > 5
+
+
+def test_a_handle_refused_before_its_device_is_known(lx, fake):
+    """As above for options that lxmfv_open refuses."""
+    fake.fake_reset()
+    h = C.c_void_p()
+    assert fake.lxmfv_open(C.byref(lx.Options(0, 96, 7, 0, 0, 0, None)), C.byref(h)) == lx.ERR_ARG
+    for name, call in _handle_calls(lx, fake, h, 96):
+        assert call() != lx.OK, name
+    assert fake.fake_launches() == 0
+    fake.lxmfv_close(h)
+    assert fake.fake_used() == 0
