@@ -198,6 +198,7 @@ struct lxmfv_pool {
     uint32_t graph_groups = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool timed = false;
+    bool opened = false;  // lxmfv_pool_open ended well: every buffer and table is there
     fe tu[LXMFV_MAX_HALF_GROUP + 1], tv[LXMFV_MAX_HALF_GROUP + 1];
     std::string err;
 };
@@ -220,6 +221,13 @@ int pfail(lxmfv_pool* p, int code, const char* fmt, ...) {
         if (e_ != cudaSuccess)                                                                \
             return pfail((p), LXMFV_ERR_CUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), \
                          __FILE__, __LINE__);                                                 \
+    } while (0)
+
+// Every call that works on the pool asks first: after an open that failed
+// part-way some buffers, host tables or the group table are missing.
+#define PNEED_OPEN(p, code)                                                 \
+    do {                                                                    \
+        if (!(p)->opened) return pfail((p), (code), "the pool is not open"); \
     } while (0)
 
 fe words8(const uint32_t w[8]) {
@@ -438,6 +446,7 @@ static int pool_open_body(const lxmfv_pool_options* opts, lxmfv_pool** out) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
     }
     if (e != cudaSuccess) return pfail(p, LXMFV_ERR_CUDA, "pool table: %s", cudaGetErrorString(e));
+    p->opened = true;
     p->err.clear();
     return LXMFV_OK;
 }
@@ -462,6 +471,7 @@ int lxmfv_pool_info(const lxmfv_pool* p, lxmfv_pool_info_t* info) {
 static int pool_submit_body(lxmfv_pool* p, const lxmfv_search_desc* d, const uint8_t* scalars, uint32_t* search_id) {
     if (!p || !d || !scalars || !search_id) return pfail(p, LXMFV_ERR_ARG, "null argument");
     if (d->lanes == 0 || d->lanes % 32) return pfail(p, LXMFV_ERR_ARG, "lanes %u: a positive multiple of 32", d->lanes);
+    PNEED_OPEN(p, LXMFV_ERR_STATE);
     const uint32_t need = d->lanes / 32;
     if (need > p->free_chunks.size())
         return pfail(p, LXMFV_ERR_OVERFLOW, "%u lanes asked, %zu free", d->lanes, p->free_chunks.size() * 32);
@@ -532,6 +542,7 @@ static int pool_submit_many_body(lxmfv_pool* p, const lxmfv_search_desc* descs, 
     if (!p || !n_admitted || (n && (!descs || !scalars || !search_ids))) return pfail(p, LXMFV_ERR_ARG, "null argument");
     *n_admitted = 0;
     if (n == 0) return LXMFV_OK;
+    PNEED_OPEN(p, LXMFV_ERR_STATE);
     // How many fit, in order; every admitted search's descriptor and scalars are checked first.
     uint64_t free_lanes = (uint64_t)p->free_chunks.size() * 32, lanes_total = 0;
     uint32_t free_slots = 0;
@@ -626,6 +637,7 @@ static int pool_submit_many_body(lxmfv_pool* p, const lxmfv_search_desc* descs, 
 
 static int pool_retire_body(lxmfv_pool* p, uint32_t search_id) {
     if (!p) return LXMFV_ERR_ARG;
+    PNEED_OPEN(p, LXMFV_ERR_STATE);
     if (search_id >= p->max_searches || !p->searches[search_id].active)
         return pfail(p, LXMFV_ERR_ARG, "search %u is not active", search_id);
     auto& s = p->searches[search_id];
@@ -644,7 +656,7 @@ static int pool_retire_body(lxmfv_pool* p, uint32_t search_id) {
 static int pool_step_body(lxmfv_pool* p, uint32_t groups) {
     if (!p) return LXMFV_ERR_ARG;
     if (groups == 0 || groups > (1u << 16)) return pfail(p, LXMFV_ERR_ARG, "groups %u: 1 .. 65536", groups);
-    if (!p->h_hit_queue) return pfail(p, LXMFV_ERR_CUDA, "the pool is not open");
+    PNEED_OPEN(p, LXMFV_ERR_CUDA);
     PCU(p, cudaSetDevice(p->device));
     if (p->queue_dirty)
         if (int rc = rebuild_queue(p)) return rc;
@@ -661,7 +673,7 @@ static int pool_step_body(lxmfv_pool* p, uint32_t groups) {
 
 int lxmfv_pool_poll(lxmfv_pool* p, lxmfv_pool_hit* hits, uint32_t cap, uint32_t* n_hits) {
     if (!p || !n_hits) return pfail(p, LXMFV_ERR_ARG, "null argument");
-    if (!p->h_hit_queue) return pfail(p, LXMFV_ERR_STATE, "the pool is not open");
+    PNEED_OPEN(p, LXMFV_ERR_STATE);
     PCU(p, cudaSetDevice(p->device));
     PCU(p, cudaStreamSynchronize(p->stream));
     // The last step's graph copied the count and the first hits to pinned memory.
@@ -685,7 +697,7 @@ int lxmfv_pool_poll(lxmfv_pool* p, lxmfv_pool_hit* hits, uint32_t cap, uint32_t*
 }
 
 uint64_t lxmfv_pool_keys_per_lane(const lxmfv_pool* p, uint32_t search_id) {
-    if (!p || search_id >= p->max_searches) return 0;
+    if (!p || search_id >= p->searches.size()) return 0;
     return p->searches[search_id].keys_per_lane;
 }
 

@@ -105,3 +105,43 @@ def test_a_handle_refused_before_its_device_is_known(lx, fake):
     assert fake.fake_launches() == 0
     fake.lxmfv_close(h)
     assert fake.fake_used() == 0
+
+
+def _pool_calls(lx, L, p):
+    scal, _ = lx.seeded_scalars(4, 0, 64)
+    d = lx.SearchDesc()
+    d.lanes = 64
+    ids, n = (C.c_uint32 * 1)(), C.c_uint32()
+    yield "submit", lambda: L.lxmfv_pool_submit(p, C.byref(d), _u8(scal), ids)
+    yield "step", lambda: L.lxmfv_pool_step(p, 1)
+    yield "poll", lambda: L.lxmfv_pool_poll(p, None, 0, C.byref(n))
+    yield "retire", lambda: L.lxmfv_pool_retire(p, 0)
+    yield "submit_many", lambda: L.lxmfv_pool_submit_many(p, C.byref(d), 1, _u8(scal), ids, C.byref(n))
+
+
+@pytest.mark.parametrize("batch", [64, 1024])
+def test_a_pool_whose_open_failed_at_any_allocation(lx, fake, batch):
+    for at in range(64):
+        fake.fake_reset()
+        fake.fake_fail_after(at)
+        p = C.c_void_p()
+        rc = fake.lxmfv_pool_open(C.byref(lx.PoolOptions(0, 256, 0, batch, 8, 0, None)), C.byref(p))
+        if fake.fake_pending():
+            assert rc == lx.OK
+            fake.fake_reset()
+            for name, call in _pool_calls(lx, fake, p):
+                assert call() == lx.OK, name
+            fake.lxmfv_pool_close(p)
+            assert fake.fake_used() == 0
+            break
+        assert rc == lx.ERR_CUDA, at
+        before = fake.fake_launches()
+        assert fake.lxmfv_pool_keys_per_lane(p, 0) == 0, at
+        for name, call in _pool_calls(lx, fake, p):
+            assert call() != lx.OK, (at, name)
+            assert fake.fake_launches() == before, (at, name)
+        fake.lxmfv_pool_close(p)
+        assert fake.fake_used() == 0, at
+    else:
+        pytest.fail("open never succeeded")
+    assert at > 9
