@@ -348,6 +348,10 @@ struct Work {
     }
 };
 
+// Private scalars do not stay in a buffer that the handle keeps (behind the
+// kernel that reads them; 2.4 MB for a whole wave, a few microseconds).
+cudaError_t wipe(lxmfv_handle* h, uint32_t* d, size_t bytes) { return cudaMemsetAsync(d, 0, bytes, h->stream); }
+
 int ensure_hits(lxmfv_handle* h, uint32_t cap) {
     if (cap <= h->hits_cap) return LXMFV_OK;
     // Grow only between launches: every queued launch has finished here.
@@ -626,6 +630,7 @@ int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_by
         }
         e = cudaGetLastError();
     }
+    if (cudaError_t w = wipe(h, d, n_bytes); e == cudaSuccess) e = w;
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "init_from_scalars: %s", cudaGetErrorString(e));
     h->initialised = true;
@@ -650,6 +655,7 @@ int lxmfv_first_public_keys(lxmfv_handle* h, const uint8_t* scalars, size_t coun
             reinterpret_cast<uint4*>(dout), ds, (uint32_t)count, t);
         e = cudaGetLastError();
     }
+    if (cudaError_t w = wipe(h, ds, count * 32); e == cudaSuccess) e = w;
     if (e == cudaSuccess) e = cudaMemcpyAsync(u_prev_cur, dout, count * 64, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "first_public_keys: %s", cudaGetErrorString(e));

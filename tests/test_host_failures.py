@@ -145,3 +145,21 @@ def test_a_pool_whose_open_failed_at_any_allocation(lx, fake, batch):
     else:
         pytest.fail("open never succeeded")
     assert at > 9
+
+
+def test_start_scalars_leave_device_memory(lx, fake):
+    """Start scalars are private keys: no copy of them stays in the handle's
+    device memory after the call that used them."""
+    fake.fake_reset()
+    lanes = 96
+    for walk in (0, 1):
+        h = C.c_void_p()
+        assert fake.lxmfv_open(C.byref(lx.Options(0, lanes, 64, 0, walk, 0, None)), C.byref(h)) == lx.OK
+        scal, _ = lx.seeded_scalars(5 + walk, 0, lanes)
+        out = np.zeros((lanes, 16), np.uint32)
+        for call in (lambda: fake.lxmfv_init_from_scalars(h, _u8(scal), C.c_size_t(32 * lanes)),
+                     lambda: fake.lxmfv_first_public_keys(h, _u8(scal), C.c_size_t(lanes), _u32(out))):
+            assert call() == lx.OK
+            for t in range(lanes):
+                assert not fake.fake_holds(bytes(scal[t]), 32), t
+        fake.lxmfv_close(h)
