@@ -38,6 +38,13 @@ extern "C" {
 #define LXMFV_ERR_RECHECK -5 /* a GPU hit failed its from-scratch CPU recheck */
 #define LXMFV_ERR_OVERFLOW -6 /* more hits than the caller's buffer holds */
 
+/* Device memory: besides walker state, hit queue and dump, a handle keeps the
+ * device buffer of its array calls (lxmfv_init, lxmfv_init_from_scalars,
+ * lxmfv_first_public_keys, lxmfv_fe_op, lxmfv_address_chain) between calls,
+ * the largest so far up to 128 MiB; a call that needs more allocates and
+ * frees its own.  lxmfv_close gives it back, and so does any allocation of
+ * the handle that would fail beside it.  Start scalars are cleared from it
+ * before the call that brought them returns. */
 typedef struct lxmfv_handle lxmfv_handle;
 
 /* Walks.  Both visit the same keys k + 8n and give the same hashes and hits.

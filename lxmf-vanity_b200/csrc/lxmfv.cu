@@ -311,6 +311,27 @@ void fill_addr_consts(lxsha::AddrConsts& ac, const uint32_t ed[8], const uint32_
 uint32_t* hit_count(const lxmfv_handle* h) { return reinterpret_cast<uint32_t*>(h->d_hit_queue); }
 lxk::Hit* hit_slots(const lxmfv_handle* h) { return reinterpret_cast<lxk::Hit*>(h->d_hit_queue) + 1; }
 
+// cudaMalloc for the handle.  Where memory is short the buffer kept for the
+// array calls goes first (no array call is running: each waits for its work);
+// an allocation that fails all the same leaves no error behind for the check
+// of the next launch.
+cudaError_t device_alloc(lxmfv_handle* h, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && h->d_work) {
+        (void)cudaGetLastError();
+        cudaFree(h->d_work);
+        h->d_work = nullptr;
+        h->work_cap = 0;
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+template <class T>
+cudaError_t device_alloc(lxmfv_handle* h, T** p, size_t bytes) {
+    return device_alloc(h, reinterpret_cast<void**>(p), bytes);
+}
+
 // Device memory for one array call (each waits for its work, so none overlap).
 // Up to kWorkKeep bytes stay with the handle: cudaMalloc and cudaFree cost 0.4
 // to 0.8 ms each on B200 and cudaFree waits for the device, against 0.5 ms for
@@ -324,13 +345,13 @@ struct Work {
     cudaError_t get(lxmfv_handle* h, size_t bytes) {
         if (bytes > kWorkKeep) {
             owned = true;
-            return cudaMalloc(&base, bytes);
+            return device_alloc(h, &base, bytes);
         }
         if (bytes > h->work_cap) {
             cudaFree(h->d_work);
             h->d_work = nullptr;
             h->work_cap = 0;
-            if (cudaError_t e = cudaMalloc(&h->d_work, bytes)) return e;
+            if (cudaError_t e = device_alloc(h, &h->d_work, bytes)) return e;
             h->work_cap = bytes;
         }
         base = h->d_work;
@@ -357,7 +378,7 @@ int ensure_hits(lxmfv_handle* h, uint32_t cap) {
     // Grow only between launches: every queued launch has finished here.
     CU(h, cudaStreamSynchronize(h->stream));
     uint8_t* q = nullptr;
-    CU(h, cudaMalloc(&q, sizeof(lxk::Hit) * ((size_t)cap + 1)));
+    CU(h, device_alloc(h, &q, sizeof(lxk::Hit) * ((size_t)cap + 1)));
     cudaError_t e;
     if (h->d_hit_queue)
         e = cudaMemcpyAsync(q, h->d_hit_queue, sizeof(lxk::Hit) * ((size_t)h->hits_cap + 1), cudaMemcpyDeviceToDevice,
@@ -383,8 +404,8 @@ int ensure_dump(lxmfv_handle* h, size_t keys) {
     h->d_dump_u = nullptr;
     h->d_dump_addr = nullptr;
     h->dump_cap_keys = 0;
-    CU(h, cudaMalloc(&h->d_dump_u, keys * 8 * sizeof(uint32_t)));
-    CU(h, cudaMalloc(&h->d_dump_addr, keys * 4 * sizeof(uint32_t)));
+    CU(h, device_alloc(h, &h->d_dump_u, keys * 8 * sizeof(uint32_t)));
+    CU(h, device_alloc(h, &h->d_dump_addr, keys * 4 * sizeof(uint32_t)));
     h->dump_cap_keys = keys;
     return LXMFV_OK;
 }
@@ -852,7 +873,7 @@ int lxmfv_peak_probe(lxmfv_handle* h, int kind, float ms, double* ops_per_s) {
     NEED_OPEN(h, LXMFV_ERR_CUDA);
     if (int rc = set_device(h)) return rc;
     uint32_t* sink = nullptr;
-    CU(h, cudaMalloc(&sink, sizeof(uint32_t)));
+    CU(h, device_alloc(h, &sink, sizeof(uint32_t)));
     const int blocks = h->sms * 8, threads = 256;
     const double per_iter = (double)blocks * threads * 16 * 8 * ((kind == 2 || kind == 5) ? 2 : 1);
     uint32_t iters = 64;

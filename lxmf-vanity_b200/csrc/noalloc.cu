@@ -5,8 +5,9 @@
 // engine with its own memory pool, a plugin that is handed device buffers and
 // must not grow the process's footprint behind the host's back), or a
 // latency-critical loop where cudaFree's implicit device synchronisation is
-// not acceptable.  lxmfv_fe_op allocates its staging and working buffers on
-// every call, so it is closed to them.
+// not acceptable.  lxmfv_fe_op allocates device memory when its buffers grow,
+// keeps it with the handle (up to 128 MiB) and allocates and frees it on every
+// call above that, so it is closed to them.
 //
 // lxmfv_fe_batch_invert_static does the same batch inversion (Montgomery's
 // trick over groups of `group` elements, as lxmfv_fe_op op 3) on buffers the

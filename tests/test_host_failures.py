@@ -163,3 +163,43 @@ def test_start_scalars_leave_device_memory(lx, fake):
             for t in range(lanes):
                 assert not fake.fake_holds(bytes(scal[t]), 32), t
         fake.lxmfv_close(h)
+
+
+def test_kept_buffers_are_given_back_when_memory_is_short(lx, fake):
+    """What a handle keeps for its array calls never stands in the way of an
+    allocation: of a dump, of hit slots, of a larger array call.  A call that
+    runs out of memory all the same fails alone."""
+    lanes, rows = 96, 1 << 18
+    nh = (C.c_uint8 * 10)()
+    big_rows = 2 * rows  # 40 MiB
+    pks, addr = np.zeros((big_rows, 64), np.uint8), np.zeros((big_rows, 16), np.uint8)
+    n = C.c_uint32()
+
+    def chain(h, count):
+        return fake.lxmfv_address_chain(h, _u8(pks), nh, _u8(addr), C.c_uint64(count))
+
+    def launch(h, **kw):
+        args = lx.make_launch_args(64, bytes(32), lx.prefix_parse("b0"), **kw)
+        return fake.lxmfv_launch(h, C.byref(args), None, 0, C.byref(n), None, None)
+
+    for what in ("dump", "hits", "array"):
+        fake.fake_reset()
+        h = C.c_void_p()
+        assert fake.lxmfv_open(C.byref(lx.Options(0, lanes, 1024, 0, 0, 0, None)), C.byref(h)) == lx.OK
+        opened = fake.fake_used()
+        scal, _ = lx.seeded_scalars(6, 0, lanes)
+        assert fake.lxmfv_init_from_scalars(h, _u8(scal), C.c_size_t(32 * lanes)) == lx.OK
+        assert chain(h, rows) == lx.OK
+        assert fake.fake_used() >= opened + 80 * rows  # kept
+        fake.fake_set_capacity(opened + 41 * (1 << 20))  # room for what comes next, but not beside the kept buffer
+        if what == "dump":
+            assert launch(h, dump_threads=8, dump_keys=1 << 16) == lx.OK  # 24 MiB
+        elif what == "hits":
+            assert launch(h, max_hits=3 << 19) == lx.OK  # 24 MiB
+        else:
+            assert chain(h, big_rows) == lx.OK
+        fake.fake_set_capacity(0)
+        assert launch(h, max_hits=1 << 28) == lx.ERR_CUDA
+        assert launch(h) == lx.OK
+        fake.lxmfv_close(h)
+        assert fake.fake_used() == 0
