@@ -76,9 +76,9 @@ NCU_PER_KEY = {
 def wide_products_per_key(walk: str, b: int) -> float:
     """32x32->64 products per key: with 8 x 32-bit limbs a field multiply is
     64 + 8 (the fold by 38), a square 36 + 8; an inversion per b keys is 20
-    batches of 76 on 9 x 30-bit limbs (fe_divsteps.h)."""
+    batches of 64 (fe_divsteps.h)."""
     mul, sqr = field_ops_per_key(walk, b)
-    return mul * 72 + sqr * 44 + 20 * 76 / b
+    return mul * 72 + sqr * 44 + 20 * 64 / b
 
 
 def parse() -> argparse.Namespace:

@@ -42,8 +42,8 @@ constexpr int kInvertThreads = 128;
 
 // Threads per group: a power of two up to 32 and the group, as long as the
 // device has an idle SM sub-partition for the next doubling.  An inversion
-// takes 16 us however long the groups are, so more warps than one per
-// sub-partition would only repeat it (a second one makes it 27 us).
+// takes 15 us however long the groups are, so more warps than one per
+// sub-partition would only repeat it (a second one makes it 23 us).
 inline uint32_t invert_threads(uint64_t groups, uint32_t group, uint32_t sms) {
     uint32_t t = 1;
     while (t < 32 && 2 * t <= group && groups * (2 * t) <= (uint64_t)sms * 128) t *= 2;

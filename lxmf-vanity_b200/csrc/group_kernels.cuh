@@ -265,7 +265,7 @@ constexpr int kPartsWarps = 16;  // warps per block (512 threads, one block per 
 // round of 1, 2, 3 or 4 warps per SM sub-partition takes 10.2, 16.7, 23.9 or
 // 31.1 us per pair (a lone warp issues at three quarters of the full rate).
 // So few lanes split until every sub-partition has a warp and the inversions
-// (16 us at least) weigh as much as the keys; full waves stay whole.
+// (15 us at least) weigh as much as the keys; full waves stay whole.
 inline uint32_t group_parts(uint64_t chunks, uint32_t m, uint32_t sms) {
     static const uint32_t kRound[5] = {0, 21, 34, 49, 64};
     const uint64_t slots = (uint64_t)sms * kPartsWarps;
