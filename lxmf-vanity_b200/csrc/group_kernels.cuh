@@ -46,6 +46,7 @@ struct GroupArgs {
     uint32_t iters;   // groups per lane in this launch
     uint32_t parts;   // warps per 32 lanes (group_parts_kernel)
     uint32_t* done;   // [lanes / 32]: warps that have finished their part; zero between launches
+    const uint4* first_words;  // [M / 4]: the first words of u of 1Q .. MQ (walks in parts from any start points)
     EmitArgs em;
     GroupTable<M> t;
 };
@@ -74,6 +75,7 @@ struct GroupArgsConst {
     uint32_t iters;
     uint32_t parts;
     uint32_t* done;
+    const uint4* first_words;
     EmitArgs em;
 };
 template <int M>
@@ -173,6 +175,32 @@ __device__ __forceinline__ fe parked_fe(const uint4* at) {
     return r;
 }
 
+// Whether a canonical u is that of a point 1Q .. MQ: by the first words, four
+// to a load, then by all (the whole table through the constant cache takes
+// 18 us at M = 512, a line's latency for every two entries; this 1.2 us: one
+// lane 0.130 -> 0.134 ms for four groups, 2,048 lanes 1.83 -> 1.86).
+template <int M, class Table>
+__device__ __forceinline__ bool table_holds(const Table& t, const uint4* __restrict__ first_words, const fe& u) {
+    bool near = false;
+#pragma unroll 8
+    for (int i = 0; i < M / 4; ++i) {
+        const uint4 w = first_words[i];
+        near |= (w.x == u.v[0]) | (w.y == u.v[0]) | (w.z == u.v[0]) | (w.w == u.v[0]);
+    }
+    bool held = false;
+    if (near) {
+#pragma unroll 1
+        for (int i = 1; i <= M; ++i) {
+            const fe x = t.u[i];
+            uint32_t d = 0;
+#pragma unroll
+            for (int w = 0; w < 8; w++) d |= x.v[w] ^ u.v[w];
+            held |= d == 0;
+        }
+    }
+    return held;
+}
+
 // `groups` groups of one lane's walk from centre (uc, vc) at walk index n
 // (the first key of the next group); emit(u, key) receives every key's
 // canonical u.  Shared by the plain walk and the pool's persistent kernel.
@@ -183,12 +211,18 @@ __device__ __forceinline__ fe parked_fe(const uint4* at) {
 // lo, hi: the part of each group to walk, the keys c +- i with lo < i <= hi
 // (and the centre where lo is 0); 0 and M: all of it.  Every part steps to
 // the next centre by itself.
+// ANY: start points of any kind (Backend::init).  A centre may then be a table
+// point up to sign, whose denominator of zero makes every inverse of its group
+// zero; so that all parts agree, each looks for its centre among all table
+// points.  Walks from clamped scalars never get there: their centres are
+// s Q with 2^251 < s, and the order of Q is above s by 2^124 keys at least.
 // The loop's registers decide its speed: at the cap of 128 ptxas's schedule of
 // the parts kernel is 7% slower than at 126 or less (4.77 against 5.14 G keys/s
 // at 37,888 lanes), so the sum u_C + A, used once per pair, waits in shared memory.
-template <int M, bool SYNC, class Table, class Emit>
+template <int M, bool SYNC, bool ANY = false, class Table, class Emit>
 __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_t groups, const Table& t,
-                                            const Emit& emit, const int lo = 0, const int hi = M) {
+                                            const Emit& emit, const int lo = 0, const int hi = M,
+                                            const uint4* first_words = nullptr) {
     __shared__ uint4 s_sum[2 * kMaxBlock];
     uint4* const sum = s_sum + threadIdx.x;
     fe pre[M + 1];
@@ -207,6 +241,7 @@ __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_
             pre[i] = acc;
             acc = fe_mul(acc, fe_add_raw(t.u[i], nu));
         }
+        if (ANY && table_holds<M>(t, first_words, uc)) acc = fe_zero();
         fe inv = fe_invert(acc);
         const uint64_t c = n + M;
         park_fe(sum, fe_canon(fe_add(uc, cA)));
@@ -341,7 +376,7 @@ static __global__ void __launch_bounds__(BLOCK, MINB) group_walk_kernel(const __
 // of it.  At G = 1024 on B200, one group: 32 lanes 0.04 ms, 2,048 lanes
 // 0.46, 100,003 lanes 19.9 (5.15 G keys/s; a whole wave 5.26); one warp per
 // chunk in blocks of 512: 15, 15 and 30 ms.
-template <int M, bool DUMP, class Args = GroupArgsFor<M>>
+template <int M, bool DUMP, bool ANY, class Args = GroupArgsFor<M>>
 static __global__ void __launch_bounds__(32 * kPartsWarps, 1) group_parts_kernel(const __grid_constant__ Args a) {
     const uint32_t lid = threadIdx.x & 31;
     const uint32_t chunks = (a.lanes + 31) / 32, parts = a.parts;
@@ -358,8 +393,8 @@ static __global__ void __launch_bounds__(32 * kPartsWarps, 1) group_parts_kernel
         const uint64_t key0 = a.ns[lane];
         uint64_t n = key0;
         const LaneEmit<DUMP> emit{a.em, lane, key0, active};
-        walk_groups<M, false>(uc, vc, n, a.iters, table_of(a), emit, part_begin(M, j, parts),
-                              part_begin(M, j + 1, parts));
+        walk_groups<M, false, ANY>(uc, vc, n, a.iters, table_of(a), emit, part_begin(M, j, parts),
+                                   part_begin(M, j + 1, parts), a.first_words);
         if (part_done(a.done + chunk, parts) && active) {
             store_fe(a.state, 0, lane, a.lanes, uc);
             store_fe(a.state, 1, lane, a.lanes, vc);

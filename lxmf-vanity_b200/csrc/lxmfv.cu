@@ -39,7 +39,7 @@ struct lxmfv_handle {
     uint32_t* d_err = nullptr;  // set by a warp-specialised launch whose wait gave up
     uint32_t* d_state = nullptr;
     uint64_t* d_ns = nullptr;
-    uint32_t* d_done = nullptr;  // grouped walk in parts: finished warps per 32 lanes
+    uint32_t* d_done = nullptr;  // grouped walk in parts: finished warps per 32 lanes; then the table's first words
     uint8_t* d_hit_queue = nullptr;  // the hit count, padded to a hit, then hits_cap hits
     uint32_t hits_cap = 0;
     uint8_t* d_work = nullptr;  // device copies of the array calls' host buffers, kept between calls
@@ -53,6 +53,7 @@ struct lxmfv_handle {
     bool timed = false;
     bool opened = false;       // lxmfv_open ended well: every buffer and table is there
     bool initialised = false;
+    bool any_start = false;    // by lxmfv_init: start points of any kind, not multiples by clamped scalars
     fe tu[LXMFV_MAX_HALF_GROUP + 1], tv[LXMFV_MAX_HALF_GROUP + 1];  // grouped walk: J, 1Q .. MQ
     std::string err;
 };
@@ -195,6 +196,10 @@ const void* walk_kernel_ptr(uint32_t walk, uint32_t batch, uint32_t block, bool 
 // counts as units of a warp, spread over all SMs.
 bool whole_waves(const lxmfv_handle* h) { return h->lanes % ((uint32_t)h->sms * 512) == 0; }
 
+// The part counters, a multiple of four, and the table's first words behind them.
+size_t done_words(const lxmfv_handle* h) { return ((size_t)h->lanes + 127) / 128 * 4; }
+const uint4* first_words(const lxmfv_handle* h) { return reinterpret_cast<const uint4*>(h->d_done + done_words(h)); }
+
 template <int B>
 void launch_xadd(lxmfv_handle* h, const lxk::WalkArgs& wa) {
     typedef void (*fn_t)(lxk::WalkArgs);
@@ -218,6 +223,7 @@ void launch_group_ws(lxmfv_handle* h, const lxk::EmitArgs& em, uint32_t iters) {
         a.g.iters = iters;
         a.g.parts = 1;
         a.g.done = nullptr;
+        a.g.first_words = nullptr;
         a.g.em = em;
         if constexpr (M <= 256) {
             for (int i = 0; i <= M; i++) {
@@ -253,9 +259,12 @@ void launch_group(lxmfv_handle* h, const lxk::EmitArgs& em, uint32_t iters) {
     const uint64_t chunks = (h->lanes + 31) / 32;
     ga.parts = lxk::group_parts(chunks, M, (uint32_t)h->sms);
     ga.done = h->d_done;
+    ga.first_words = first_words(h);
     if (!h->low_regs && (ga.parts > 1 || !whole_waves(h))) {
         const unsigned grid = (unsigned)std::min<uint64_t>(h->sms, chunks * ga.parts);
-        const fn_t fn = em.dump_lanes > 0 ? (fn_t)lxk::group_parts_kernel<M, true> : (fn_t)lxk::group_parts_kernel<M, false>;
+        const bool any = h->any_start && ga.parts > 1;
+        const fn_t fn = (fn_t)(em.dump_lanes > 0 ? any ? lxk::group_parts_kernel<M, true, true> : lxk::group_parts_kernel<M, true, false>
+                                                 : any ? lxk::group_parts_kernel<M, false, true> : lxk::group_parts_kernel<M, false, false>);
         fn<<<grid, 32 * lxk::kPartsWarps, 0, h->stream>>>(ga);
         return;
     }
@@ -480,6 +489,12 @@ int build_group_table(lxmfv_handle* h) {
                                         h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     }
+    if (e == cudaSuccess) {
+        uint32_t first[LXMFV_MAX_HALF_GROUP];
+        for (uint32_t i = 0; i < m; i++) first[i] = h->tu[i + 1].v[0];
+        e = cudaMemcpyAsync(h->d_done + done_words(h), first, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    }
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "group table: %s", cudaGetErrorString(e));
     return LXMFV_OK;
 }
@@ -574,8 +589,9 @@ int lxmfv_open(const lxmfv_options* opts, lxmfv_handle** out) {
     }
     CU(h, cudaMalloc(&h->d_state, (size_t)h->lanes * 32 * sizeof(uint32_t)));
     CU(h, cudaMalloc(&h->d_ns, (size_t)h->lanes * sizeof(uint64_t)));
-    CU(h, cudaMalloc(&h->d_done, (size_t)((h->lanes + 31) / 32) * sizeof(uint32_t)));
-    CU(h, cudaMemsetAsync(h->d_done, 0, (size_t)((h->lanes + 31) / 32) * sizeof(uint32_t), h->stream));
+    const size_t done_bytes = (done_words(h) + LXMFV_MAX_HALF_GROUP) * sizeof(uint32_t);
+    CU(h, cudaMalloc(&h->d_done, done_bytes));
+    CU(h, cudaMemsetAsync(h->d_done, 0, done_bytes, h->stream));
     CU(h, cudaMemsetAsync(h->d_state, 0, (size_t)h->lanes * 32 * sizeof(uint32_t), h->stream));
     CU(h, cudaMemsetAsync(h->d_ns, 0, (size_t)h->lanes * sizeof(uint64_t), h->stream));
     if (int rc = ensure_hits(h, 4096)) return rc;
@@ -624,6 +640,7 @@ int lxmfv_init(lxmfv_handle* h, const uint32_t* u_prev_cur, size_t n_words) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "init: %s", cudaGetErrorString(e));
     h->initialised = true;
+    h->any_start = true;
     h->err.clear();
     return LXMFV_OK;
 }
@@ -655,6 +672,7 @@ int lxmfv_init_from_scalars(lxmfv_handle* h, const uint8_t* scalars, size_t n_by
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return fail(h, LXMFV_ERR_CUDA, "init_from_scalars: %s", cudaGetErrorString(e));
     h->initialised = true;
+    h->any_start = false;
     h->err.clear();
     return LXMFV_OK;
 }
