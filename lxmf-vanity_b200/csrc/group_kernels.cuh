@@ -324,16 +324,18 @@ __device__ __forceinline__ int part_begin(uint32_t m, uint32_t j, uint32_t parts
 
 // A warp has walked its part of a chunk.  True for the last of the S
 // warps to come here, the one that stores the chunk's new state: by then the
-// others have read the old one.
+// others have read the old one.  The count orders those reads before the
+// store: released by each warp, acquired by the last, and passed on to and from
+// the other lanes by the warp barriers.
 __device__ __forceinline__ bool part_done(uint32_t* done, uint32_t parts) {
     if (parts == 1) return true;
     uint32_t before = 0;
     __syncwarp();
     if ((threadIdx.x & 31) == 0) {
-        __threadfence();
-        before = atomicAdd(done, 1u);
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(__cvta_generic_to_global(done)) : "memory");
         if (before == parts - 1) *done = 0;  // for the next launch
     }
+    __syncwarp();
     return __shfl_sync(0xffffffffu, before, 0) == parts - 1;
 }
 
