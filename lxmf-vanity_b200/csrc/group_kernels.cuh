@@ -156,11 +156,12 @@ static __global__ void __launch_bounds__(128) group_init_kernel(uint32_t* state,
 
 // One field element per thread in shared memory, out of the registers' way.
 // The load is volatile: it stays where it is used.
-constexpr int kMaxBlock = 512;
+template <int BLOCK>
 __device__ __forceinline__ void park_fe(uint4* at, const fe& x) {
     at[0] = make_uint4(x.v[0], x.v[1], x.v[2], x.v[3]);
-    at[kMaxBlock] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
+    at[BLOCK] = make_uint4(x.v[4], x.v[5], x.v[6], x.v[7]);
 }
+template <int BLOCK>
 __device__ __forceinline__ fe parked_fe(const uint4* at) {
     const uint32_t p = (uint32_t)__cvta_generic_to_shared(at);
     fe r;
@@ -170,7 +171,7 @@ __device__ __forceinline__ fe parked_fe(const uint4* at) {
                  : "memory");
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
-                 : "r"(p + 16 * kMaxBlock)
+                 : "r"(p + 16 * BLOCK)
                  : "memory");
     return r;
 }
@@ -216,14 +217,16 @@ __device__ __forceinline__ bool table_holds(const Table& t, const uint4* __restr
 // zero; so that all parts agree, each looks for its centre among all table
 // points.  Walks from clamped scalars never get there: their centres are
 // s Q with 2^251 < s, and the order of Q is above s by 2^124 keys at least.
-// The loop's registers decide its speed: at the cap of 128 ptxas's schedule of
-// the parts kernel is 7% slower than at 126 or less (4.77 against 5.14 G keys/s
-// at 37,888 lanes), so the sum u_C + A, used once per pair, waits in shared memory.
-template <int M, bool SYNC, bool ANY = false, class Table, class Emit>
+// The loop takes 126 to 128 registers, the cap, in all its kernels; with the
+// sum u_C + A among them, and -u_C or -v_C, ptxas schedules around the cap and
+// the parts kernel loses 7% (4.71-4.77 against 5.12-5.14 G keys/s at 37,888
+// lanes).  So the sum, used once per pair, waits in shared memory, 32 bytes per
+// thread of the block.
+template <int M, int BLOCK, bool SYNC, bool ANY = false, class Table, class Emit>
 __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_t groups, const Table& t,
                                             const Emit& emit, const int lo = 0, const int hi = M,
                                             const uint4* first_words = nullptr) {
-    __shared__ uint4 s_sum[2 * kMaxBlock];
+    __shared__ uint4 s_sum[2 * BLOCK];
     uint4* const sum = s_sum + threadIdx.x;
     fe pre[M + 1];
     fe cA = fe_zero();
@@ -244,7 +247,7 @@ __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_
         if (ANY && table_holds<M>(t, first_words, uc)) acc = fe_zero();
         fe inv = fe_invert(acc);
         const uint64_t c = n + M;
-        park_fe(sum, fe_canon(fe_add(uc, cA)));
+        park_fe<BLOCK>(sum, fe_canon(fe_add(uc, cA)));
         fe vnext = vc;
 #pragma unroll 1
         for (int k = hi; k >= lo; --k) {
@@ -255,7 +258,7 @@ __device__ __forceinline__ void walk_groups(fe& uc, fe& vc, uint64_t& n, uint32_
                 invi = fe_mul(inv, pre[i]);
                 inv = fe_mul(inv, fe_add_raw(tu, nu));
             }
-            const fe s = fe_add_raw(parked_fe(sum), tu);
+            const fe s = fe_add_raw(parked_fe<BLOCK>(sum), tu);
             const fe lp = fe_mul(fe_sub(tv, vc), invi);
             const fe up = fe_sub_canon(fe_sqr(lp), s);  // C + T_i (for i = 0: the next centre C + J)
             fe um;
@@ -364,7 +367,7 @@ static __global__ void __launch_bounds__(BLOCK, MINB) group_walk_kernel(const __
     const uint64_t key0 = a.ns[lane];
     uint64_t n = key0;
     const LaneEmit<DUMP> emit{a.em, lane, key0, active};
-    walk_groups<M, SYNC>(uc, vc, n, a.iters, table_of(a), emit);
+    walk_groups<M, BLOCK, SYNC>(uc, vc, n, a.iters, table_of(a), emit);
     if (active) {
         store_fe(a.state, 0, lane, a.lanes, uc);
         store_fe(a.state, 1, lane, a.lanes, vc);
@@ -395,8 +398,8 @@ static __global__ void __launch_bounds__(32 * kPartsWarps, 1) group_parts_kernel
         const uint64_t key0 = a.ns[lane];
         uint64_t n = key0;
         const LaneEmit<DUMP> emit{a.em, lane, key0, active};
-        walk_groups<M, false, ANY>(uc, vc, n, a.iters, table_of(a), emit, part_begin(M, j, parts),
-                                   part_begin(M, j + 1, parts), a.first_words);
+        walk_groups<M, 32 * kPartsWarps, false, ANY>(uc, vc, n, a.iters, table_of(a), emit, part_begin(M, j, parts),
+                                                      part_begin(M, j + 1, parts), a.first_words);
         if (part_done(a.done + chunk, parts) && active) {
             store_fe(a.state, 0, lane, a.lanes, uc);
             store_fe(a.state, 1, lane, a.lanes, vc);

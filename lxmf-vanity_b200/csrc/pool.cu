@@ -129,8 +129,8 @@ static __global__ void __launch_bounds__(32 * kPoolWarps, 1) pool_walk_kernel(co
         fe vc = load_fe(a.state, 1, lane, a.capacity);
         uint64_t n = a.ns[lane];
         const PoolEmit emit{s_ac[warp], a.hit_count, a.hits, a.max_hits, search, entry.z + lid, a.one};
-        walk_groups<M, false>(uc, vc, n, a.groups, pool_table(a.t), emit, part_begin(M, j, parts),
-                              part_begin(M, j + 1, parts));
+        walk_groups<M, 32 * kPoolWarps, false>(uc, vc, n, a.groups, pool_table(a.t), emit, part_begin(M, j, parts),
+                                               part_begin(M, j + 1, parts));
         if (part_done(a.done + chunk, parts)) {
             store_fe(a.state, 0, lane, a.capacity, uc);
             store_fe(a.state, 1, lane, a.capacity, vc);
