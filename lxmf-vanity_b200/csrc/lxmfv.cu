@@ -31,6 +31,7 @@ struct lxmfv_handle {
     bool own_stream = false;
     uint32_t walk = LXMFV_WALK_GROUP;
     uint32_t lanes = 0;
+    uint32_t parts = 1;   // grouped walk: warps per 32 lanes (group_parts)
     uint32_t batch = 64;  // keys per inversion: B (x-only walk) or G = 2M (grouped walk)
     uint32_t block = 256;
     bool sync = false;    // grouped walk: block barrier after each group
@@ -257,7 +258,7 @@ void launch_group(lxmfv_handle* h, const lxk::EmitArgs& em, uint32_t iters) {
     // Other counts than whole waves in parts; the register-capped build is
     // always its own shape.
     const uint64_t chunks = (h->lanes + 31) / 32;
-    ga.parts = lxk::group_parts(chunks, M, (uint32_t)h->sms);
+    ga.parts = h->parts;
     ga.done = h->d_done;
     ga.first_words = first_words(h);
     if (!h->low_regs && (ga.parts > 1 || !whole_waves(h))) {
@@ -587,6 +588,8 @@ int lxmfv_open(const lxmfv_options* opts, lxmfv_handle** out) {
             return fail(h, LXMFV_ERR_CUDA, "walk kernel cannot be resident (batch %u, block %u)", h->batch, h->block);
         h->lanes = o.lanes ? o.lanes : (uint32_t)(h->sms * per_sm) * h->block;
     }
+    if (h->walk == LXMFV_WALK_GROUP && !h->ws)
+        h->parts = lxk::group_parts(((uint64_t)h->lanes + 31) / 32, h->batch / 2, (uint32_t)h->sms);
     CU(h, cudaMalloc(&h->d_state, (size_t)h->lanes * 32 * sizeof(uint32_t)));
     CU(h, cudaMalloc(&h->d_ns, (size_t)h->lanes * sizeof(uint64_t)));
     const size_t done_bytes = (done_words(h) + LXMFV_MAX_HALF_GROUP) * sizeof(uint32_t);
