@@ -58,7 +58,7 @@ def field_ops_per_key(walk: str, b: int) -> tuple[float, float]:
     return (5 * m + 2) / b, (2 * m + 1) / b
 
 
-# Per key, from ncu captures of each kernel on a small case (profiles/pipe_counts_plain_search.md):
+# Per key, from ncu captures of each kernel on a small case:
 #   alu: ALU-pipe lane operations (the binding pipe): sm__inst_executed_pipe_alu.sum x 32 / keys;
 #   imad: IMAD-class instructions per key: sm__inst_executed_pipe_fmaheavy.sum x 32 / keys, the pipe that
 #        executes IMAD, IMAD.HI, IMAD.WIDE and IMAD.X (these kernels run no floating point);

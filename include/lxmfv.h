@@ -188,10 +188,10 @@ void lxmfv_close(lxmfv_handle* h);
  * (GpuSearch, mod.rs:86-174) and starts more processes to search more
  * (fleet.sh).  Searches with different prefixes, aspects and identities are
  * admitted into a device-resident pool of walker lanes, walked together by a
- * persistent kernel that takes 32-lane chunks from a device work queue, and
- * retired as their hits come in.  Every step advances every active lane by
+ * persistent kernel that takes 32-lane chunks, or parts of their groups, from a
+ * device work queue, and retired as their hits come in.  Every step advances every active lane by
  * the same number of keys, so a search's hits do not depend on the rest of
- * the pool.  A step is a CUDA graph (reset, persistent kernel, hit read-back)
+ * the pool.  A step is a CUDA graph (persistent kernel, hit read-back)
  * captured once per step length. */
 typedef struct lxmfv_pool lxmfv_pool;
 

@@ -7,9 +7,11 @@
 // raised by four doublings.  64 x 7 M + 16 M + 16 S + one inversion per start
 // point, where a Montgomery ladder takes 253 x (5 M + 4 S) and its inversion.
 //
-// As the ladder, no branch and no address depends on a scalar: every digit
-// reads all eight entries of its window, at one address per warp, from shared
-// memory, and keeps one by selects (about a fifth of the addition's time).
+// No address and no choice of an entry depends on a scalar: every digit reads
+// all eight entries of its window, at one address per warp, from shared memory,
+// and keeps one by selects (about a fifth of the addition's time).  What is
+// left, as in a ladder on the same field functions, are their branches on a
+// last carry, taken below 2^-21 of the time.
 #pragma once
 #include <cstdint>
 
@@ -126,8 +128,10 @@ __device__ __forceinline__ fe shfl_xor_fe(const fe& x, int m) {
     return r;
 }
 
-// s Q for s < 2^255 (8 little-endian words), by `threads` threads (a power of
-// two; thread t takes the windows t, t + threads, ...): every one gets it.
+// s Q for s <= 0x77...7, 64 sevens (8 little-endian words; above that the sum
+// below leaves 256 bits; a clamped scalar over 8 and the group's half are below
+// 2^252 + 2^10), by `threads` threads (a power of two; thread t takes the windows
+// t, t + threads, ...): every one gets it.
 __device__ __forceinline__ EdPoint comb_mul(const uint32_t s[8], const uint4* table, uint32_t t, uint32_t threads) {
     // s + 8 (1 + 16 + ... + 16^63): its nibbles less 8 are signed digits of s.
     uint32_t n[8], carry = 0;

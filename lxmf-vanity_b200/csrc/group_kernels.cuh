@@ -13,7 +13,7 @@
 // C + T_i and C - T_i share the denominator u_T - u_C, so one batch inversion
 // (Montgomery's trick) over the M denominators and the step to the next
 // centre, C' = C + J with J = 2M Q, serves all 2M keys.  Per group:
-// (5M + 4) M + (2M + 1) S and one inversion, about 2.5 M + 1 S per key,
+// (5M + 2) M + (2M + 1) S and one inversion, about 2.5 M + 1 S per key,
 // against 8 M + 4 S for the x-only walk (G = B = 128).  The lane's local
 // buffer holds only the M prefix products (the denominators are recomputed
 // from the table on the way back).
