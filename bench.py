@@ -64,12 +64,12 @@ def field_ops_per_key(walk: str, b: int) -> tuple[float, float]:
 #        executes IMAD, IMAD.HI, IMAD.WIDE and IMAD.X (these kernels run no floating point);
 #   inst: all instructions (smsp__inst_executed.sum x 32 / keys); dram_bytes: DRAM read + write.
 NCU_PER_KEY = {
-    ("group", 1024): {"alu": 2844, "imad": 1902, "inst": 4939, "dram_bytes": 31.4},
-    ("group", 512): {"alu": 2850, "imad": 1912, "inst": 4955, "dram_bytes": 30.5},
-    ("group", 256): {"alu": 2862, "imad": 1932, "inst": 4988, "dram_bytes": 29.3},
-    ("group", 64): {"alu": 2938, "imad": 2055, "inst": 5191, "dram_bytes": 10.4},
-    ("xadd", 128): {"alu": 3146, "imad": 2435, "inst": 5794, "dram_bytes": 121.4},
-    ("xadd", 64): {"alu": 3203, "imad": 2503, "inst": 5921, "dram_bytes": 114.5},
+    ("group", 1024): {"alu": 2836, "imad": 1908, "inst": 4937, "dram_bytes": 31.0},
+    ("group", 512): {"alu": 2842, "imad": 1917, "inst": 4952, "dram_bytes": 30.6},
+    ("group", 256): {"alu": 2854, "imad": 1935, "inst": 4982, "dram_bytes": 29.3},
+    ("group", 64): {"alu": 2924, "imad": 2046, "inst": 5167, "dram_bytes": 10.4},
+    ("xadd", 128): {"alu": 3125, "imad": 2444, "inst": 5782, "dram_bytes": 121.5},
+    ("xadd", 64): {"alu": 3180, "imad": 2501, "inst": 5896, "dram_bytes": 114.5},
 }
 
 

@@ -299,7 +299,8 @@ constexpr int kPartsWarps = 16;  // warps per block (512 threads, one block per 
 // S for `chunks` chunks of 32 lanes on `sms` SMs: the one with the smallest
 // predicted time, (ceil(M/S) + 1.8) x (full rounds of 16 warps per SM + the
 // last round's share).  Measured on B200: an inversion with the step to
-// the next centre takes as long as 1.8 pairs of keys at any occupancy, and a
+// the next centre takes as long as 1.8 pairs of keys at any occupancy (on 30-bit
+// limbs; 8% less now, and the rule not refitted), and a
 // round of 1, 2, 3 or 4 warps per SM sub-partition takes 10.2, 16.7, 23.9 or
 // 31.1 us per pair (a lone warp issues at three quarters of the full rate).
 // So few lanes split until every sub-partition has a warp and the inversions
